@@ -10,6 +10,7 @@
 // The header also compiles as plain C++ for the host, where the tests check
 // every function against the compare it replaces.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -114,6 +115,146 @@ MPRW_FB double ih12_normal(unsigned long long sum) {
                                ((unsigned long long)(e + 991) << 52) |  // 991 = 1023 - 32
                                ((m << (52 - e)) & 0x000FFFFFFFFFFFFFULL);
   return from_bits(m ? b : 0ULL);
+}
+
+// ---- division and square root on the integer pipe ---------------------------
+// a / b and sqrt(x), correctly rounded to nearest, for FP64 operands: the same
+// bits as the FP64 operators, which IEEE-754 rounds the same way.  An FP64
+// division or square root is a chain of about nine dependent FP64 instructions,
+// each holding GB300's FP64 pipe for 16 clocks per warp; here the FP64 pipe is
+// not used at all.  The quotient (root) is built in three digits of a long
+// division (digit-by-digit root): each digit is the running remainder's top 32
+// bits times a 32-bit reciprocal (inverse root) taken from the FP32
+// approximation, the remainder is carried exactly in 64-bit wrapping integers,
+// and the last remainder decides the final unit.  With the reciprocal within
+// 2^-20 relative (the FP32 approximations are within 2^-21.5, truncated
+// operand included) the digits leave the 54-bit result at most one unit off
+// before that last step; the host test runs both with the approximation
+// perturbed either way.  A quotient of two 53-bit significands, and a root of
+// one, never lies midway between two of them, so the extra (54th) bit alone
+// rounds to nearest.
+// Operands or quotients outside the plain normal range (zeros, subnormals,
+// infinities, NaN, negative radicands, exponents at the ends) take the
+// operator: div_plain / sqrt_plain tell.
+#if !defined(__CUDA_ARCH__)
+// the host stands in for the two FP32 approximations, off by this many ulps
+inline int &host_approx_ulps() {
+  static int k = 0;
+  return k;
+}
+inline float host_approx(float r) {
+  unsigned u;
+  std::memcpy(&u, &r, 4);
+  u += (unsigned)host_approx_ulps();
+  std::memcpy(&r, &u, 4);
+  return r;
+}
+#endif
+// bits of the FP32 approximations 1/f and 1/sqrt(f), f given by its bits
+MPRW_FB unsigned rcp_bits(unsigned f) {
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(f)));
+  return __float_as_uint(r);
+#else
+  float x, r;
+  std::memcpy(&x, &f, 4);
+  r = host_approx(1.0f / x);
+  unsigned u;
+  std::memcpy(&u, &r, 4);
+  return u;
+#endif
+}
+MPRW_FB unsigned rsqrt_bits(unsigned f) {
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(f)));
+  return __float_as_uint(r);
+#else
+  float x, r;
+  std::memcpy(&x, &f, 4);
+  r = host_approx((float)(1.0 / std::sqrt((double)x)));
+  unsigned u;
+  std::memcpy(&u, &r, 4);
+  return u;
+#endif
+}
+// an approximation in (1/2, 1), by its bits, as a 31-bit fraction (its rounding
+// kept from reaching either end)
+MPRW_FB int frac31(unsigned r) {
+  r = r < 0x3F000000u ? 0x3F000000u : (r > 0x3F7FFFFFu ? 0x3F7FFFFFu : r);
+  return (int)((r << 7) & 0x3FFFFF80u) | 0x40000000;
+}
+// (a * b) >> 32 of a signed and an unsigned 31-bit factor
+MPRW_FB int mulhi_s(int a, int b) {
+#if defined(__CUDA_ARCH__)
+  return __mulhi(a, b);
+#else
+  return (int)(((long long)a * (long long)b) >> 32);
+#endif
+}
+
+// both operands normal, and the quotient and its half normal too
+MPRW_FB bool div_plain(double a, double b) {
+  const unsigned ea = ((unsigned)(bits(a) >> 52) & 0x7FFu) - 1u, eb = ((unsigned)(bits(b) >> 52) & 0x7FFu) - 1u;
+  return (ea < 2046u) & (eb < 2046u) & (ea - eb + 1020u < 2042u);
+}
+// a / b * 2^-scale, scale 0 or 1, for div_plain operands
+MPRW_FB double div_core(double a, double b, int scale) {
+  const unsigned long long ba = bits(a), bb = bits(b);
+  unsigned long long ma = (ba & 0x000FFFFFFFFFFFFFULL) | 0x0010000000000000ULL;
+  const unsigned long long mb = (bb & 0x000FFFFFFFFFFFFFULL) | 0x0010000000000000ULL;
+  int e = (int)((ba >> 52) & 0x7FF) - (int)((bb >> 52) & 0x7FF) + 1022 - scale;
+  // quotient in [1, 2): shift a left when its significand is the smaller
+  const bool less = ma < mb;
+  ma <<= less ? 1 : 0;
+  e -= less ? 1 : 0;
+  // rho = 2^52 / mb in (1/2, 1): the divisor rounded up to 24 bits, so the
+  // approximation stays below 1; q31 = rho 2^31
+  const int q31 = frac31(rcp_bits(0x3F800001u + (unsigned)((bb >> 29) & 0x7FFFFFULL)));
+  // ma / mb = ma * rho * 2^-52.  Digits: 2^-23, 2^-43, 2^-53
+  const int q1 = (int)((unsigned)mulhi_s((int)(ma >> 23), q31) >> 5);          // ma (54 bits) -> 24 bits
+  const long long r1 = (long long)((ma << 23) - (unsigned long long)(unsigned)q1 * mb);  // |r1| < 2^57
+  const int q2 = mulhi_s((int)(r1 >> 26), q31) >> 5;
+  const long long r2 = (long long)((unsigned long long)r1 << 20) - (long long)q2 * (long long)mb;  // |r2| < 2^57
+  const int q3 = mulhi_s((int)(r2 >> 26), q31) >> 15;
+  const long long r3 = (long long)((unsigned long long)r2 << 10) - (long long)q3 * (long long)mb;
+  unsigned long long q = ((unsigned long long)(unsigned)q1 << 30) + (unsigned long long)((long long)q2 * 1024 + q3);
+  q -= (r3 < 0) ? 1ULL : 0ULL;
+  q += (r3 >= (long long)mb) ? 1ULL : 0ULL;
+  // q = floor(a/b 2^53), 54 bits: round on its last bit; the carry of 1.11..1
+  // moves into the exponent
+  const unsigned long long m = (q + 1ULL) >> 1;
+  return from_bits(((ba ^ bb) & 0x8000000000000000ULL) | (((unsigned long long)(unsigned)e << 52) + m));
+}
+
+// x normal and positive
+MPRW_FB bool sqrt_plain(double x) { return bits(x) - 0x0010000000000000ULL < 0x7FE0000000000000ULL; }
+// sqrt(x) for sqrt_plain x
+MPRW_FB double sqrt_core(double x) {
+  const unsigned long long b = bits(x);
+  // x = m 4^k, m in [1, 4): M = m 2^52, 54 bits
+  const unsigned odd = (unsigned)(b >> 52) & 1u;  // biased exponent odd: 1023 + even, m in [1, 2)
+  const unsigned long long M = ((b & 0x000FFFFFFFFFFFFFULL) | 0x0010000000000000ULL) << (odd ? 0 : 1);
+  const unsigned e = ((unsigned)(b >> 52) + 1023u) >> 1;  // biased exponent of the root (even: m doubled)
+  // rho = 1/sqrt(m) in (1/2, 1): m rounded up to its FP32 neighbour
+  const int q31 = frac31(rsqrt_bits((odd ? 0x3F800001u : 0x40000001u) + (unsigned)((b >> 29) & 0x7FFFFFULL)));
+  // root = s1 2^-23 + d2 2^-43 + d3 2^-53
+  const unsigned s1 = (unsigned)mulhi_s((int)(M >> 23), q31) >> 5;              // m rho, 24 bits
+  const long long r1 = (long long)(M - ((unsigned long long)s1 * s1 << 6));     // units 2^-52
+  const int d2 = mulhi_s((int)(r1 >> 4), q31) >> 5;
+  const long long t1 = (long long)((unsigned long long)s1 << 21);
+  const long long r2 = (long long)((unsigned long long)r1 << 34) - (long long)d2 * (t1 + d2);  // units 2^-86
+  const int d3 = mulhi_s((int)(r2 >> 18), q31) >> 15;
+  const unsigned long long s2 = ((unsigned long long)s1 << 20) + (unsigned long long)(long long)d2;
+  const long long r3 = (long long)((unsigned long long)r2 << 20) -
+                       (long long)d3 * ((long long)(s2 << 11) + d3);            // units 2^-106
+  unsigned long long q = (s2 << 10) + (unsigned long long)(long long)d3;
+  const bool up = r3 > (long long)(2 * q);
+  q -= (r3 < 0) ? 1ULL : 0ULL;
+  q += up ? 1ULL : 0ULL;
+  const unsigned long long m = (q + 1ULL) >> 1;
+  return from_bits(((unsigned long long)(e - 1u) << 52) + m);
 }
 
 }  // namespace fb

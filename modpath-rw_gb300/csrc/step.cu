@@ -78,6 +78,23 @@ template <typename R>
 __device__ __forceinline__ bool pos_lt(R a, R b) { return a < b; }
 template <>
 __device__ __forceinline__ bool pos_lt<double>(double a, double b) { return fb::pos_lt(a, b); }
+// Square root and quotient of the FP64 kernels: on the integer pipe (the same
+// bits; the operator, out of line, outside the plain normal range).  A pass
+// takes about six roots and four quotients per warp, eight FP64 instructions
+// each, on the pipe that bounds the kernel (78 % active before).  The first
+// 10-day interval of 200,000 particles in the lognormal slab: 6.80 -> 6.20 ms,
+// FP64 pipe 70 %; with the exit solves' operands in shared memory 5.62 ms, 75 %.
+__device__ __noinline__ double sqrt_op(double x) { return sqrt(x); }
+__device__ __noinline__ double div_op(double a, double b) { return a / b; }
+template <typename R>
+__device__ __forceinline__ R sqrt_r(R x) { return sqrt(x); }
+template <>
+__device__ __forceinline__ double sqrt_r<double>(double x) {
+  return fb::sqrt_plain(x) ? fb::sqrt_core(x) : sqrt_op(x);
+}
+__device__ __forceinline__ double div_r(double a, double b) {
+  return fb::div_plain(a, b) ? fb::div_core(a, b, 0) : div_op(a, b);
+}
 using fb::eq_any;
 using fb::lt_any;
 using fb::past_end;
@@ -182,7 +199,7 @@ __device__ __forceinline__ void random_displacement(const Lane<R> &F, int ndim, 
   R aL = F(F_AL), aT = F(F_AT), dm = F(F_DM), tr = F(F_2R);
   R aTH = aT;
   if constexpr (AXI) {
-    const R vnorm = sqrt(vpx * vpx + vpy * vpy + vpz * vpz);
+    const R vnorm = sqrt_r(vpx * vpx + vpy * vpy + vpz * vpz);
     R cosinesq = zero;
     if (vnorm > zero) cosinesq = vpz * vpz / vnorm;
     aL = aL + cosinesq * (F(F_ALV) - aL);
@@ -198,9 +215,9 @@ __device__ __forceinline__ void random_displacement(const Lane<R> &F, int ndim, 
     if (sizeof(R) == 8 ? above0(n2) : n2 > zero) {
       R inv = rsqrt(n2);
       R nrm = n2 * inv;
-      R sL = sqrt(tr * fma(aL, nrm, dm));
-      R sT = sqrt(tr * fma(aT, nrm, dm));
-      R sTH = AXI ? sqrt(tr * fma(aTH, nrm, dm)) : sT;
+      R sL = sqrt_r(tr * fma(aL, nrm, dm));
+      R sT = sqrt_r(tr * fma(aT, nrm, dm));
+      R sTH = AXI ? sqrt_r(tr * fma(aTH, nrm, dm)) : sT;
       R sLi = sL * inv;
       B11 = vx * sLi;
       B21 = vy * sLi;
@@ -231,8 +248,8 @@ __device__ __forceinline__ void random_displacement(const Lane<R> &F, int ndim, 
     if (n2 > zero) {
       R inv = rsqrt(n2);
       R nrm = n2 * inv;
-      R sLi = sqrt(tr * fma(aL, nrm, dm)) * inv;
-      R sTi = sqrt(tr * fma(aTH, nrm, dm)) * inv;
+      R sLi = sqrt_r(tr * fma(aL, nrm, dm)) * inv;
+      R sTi = sqrt_r(tr * fma(aTH, nrm, dm)) * inv;
       B11 = v1 * sLi;
       B21 = v2 * sLi;
       B12 = -v2 * sTi;
@@ -248,7 +265,7 @@ __device__ __forceinline__ void random_displacement(const Lane<R> &F, int ndim, 
     R v1 = tril(F, F_VB + 8 * d1, x, y, z, xy, xz, yz, xyz);
     R nrm = fabs(v1);
     R B11 = zero;
-    if (nrm > zero) B11 = sqrt(tr * fma(aL, nrm, dm));
+    if (nrm > zero) B11 = sqrt_r(tr * fma(aL, nrm, dm));
     R r1, r2, r3;
     Normals<R>::draw(1, seed, id, ctr, r1, r2, r3);
     bx = zero; by = zero; bz = zero;
@@ -324,13 +341,14 @@ __device__ __forceinline__ bool quad_axis(R npos, R pos, R d, R v, R divD, R dB,
 
 // quad_axis in FP64 with its tests against 0 and 1 and its step compare on
 // the integer pipe (the same decisions, see above).
-__device__ __forceinline__ bool quad_axis_f64(double npos, double pos, double d, double v, double divD, double dB,
+// `high`: the step leaves through the axis's upper face.
+__device__ __forceinline__ bool quad_axis_f64(bool high, double pos, double d, double v, double divD, double dB,
                                               int faceLo, int faceHi, double dt, double &dtaxis, int &exitAxis,
                                               int &exitFace, double &dtout) {
   using R = double;
   const R zero = R(0), one = R(1);
   R dI;
-  if (above1(npos)) {
+  if (high) {
     dI = d * (one - pos);
     exitAxis = faceHi;
   } else {
@@ -345,27 +363,45 @@ __device__ __forceinline__ bool quad_axis_f64(double npos, double pos, double d,
   R A = v + divD, B = dB;
   R arg = B * B + R(4) * dI * A;
   if (nonneg(arg) && !is0(A)) {
-    R zs = sqrt(arg);
-    R z1, z2;
-    z1 = (-B + zs) / (R(2) * A);
-    z2 = (-B - zs) / (R(2) * A);
-    const bool p1 = above0(z1), p2 = above0(z2);
-    if (p1 || p2) {
-      R zm = (p1 && p2) ? (pos_lt(z1, z2) ? z1 : z2) : (p1 ? z1 : z2);
+    const R zs = sqrt_r(arg);
+    // roots z1 = n1 / (2A), z2 = n2 / (2A), n1 >= n2: the smaller positive
+    // one is n2's for A > 0 and n1's for A < 0 when that is positive, else the
+    // other; one division instead of two
+    const R n1 = -B + zs, n2 = -B - zs;
+    const bool pa = above0(A);
+    const R na = pa ? n2 : n1, nb = pa ? n1 : n2;
+    const bool fa = pa ? above0(na) : below0(na), fbk = pa ? above0(nb) : below0(nb);
+    const R nm = fa ? na : nb;
+    if ((fa || fbk) && fb::div_plain(nm, A)) {
+      const R zm = fb::div_core(nm, A, 1);
       dtaxis = zm * zm;
       if (is0(dtaxis)) {
         exitFace = exitAxis;
         dtout = 0.0;
         return true;
       }
-    } else if (is0(z1) || is0(z2)) {
-      exitFace = exitAxis;
-      dtout = 0.0;
-      return true;
+    } else {
+      // no positive numerator, or a quotient outside the plain range: both
+      // roots as written
+      const R z1 = div_op(n1, R(2) * A), z2 = div_op(n2, R(2) * A);
+      const bool p1 = above0(z1), p2 = above0(z2);
+      if (p1 || p2) {
+        R zm = (p1 && p2) ? (pos_lt(z1, z2) ? z1 : z2) : (p1 ? z1 : z2);
+        dtaxis = zm * zm;
+        if (is0(dtaxis)) {
+          exitFace = exitAxis;
+          dtout = 0.0;
+          return true;
+        }
+      } else if (is0(z1) || is0(z2)) {
+        exitFace = exitAxis;
+        dtout = 0.0;
+        return true;
+      }
     }
   } else if (is0(A)) {
     if (!is0(B)) {
-      R q = dI / B;
+      R q = div_r(dI, B);
       dtaxis = q * q;
       if (is0(dtaxis)) {
         exitFace = exitAxis;
@@ -382,192 +418,263 @@ __device__ __forceinline__ bool quad_axis_f64(double npos, double pos, double d,
 // Newton-Raphson (:1895-2554).  Both run in FP64 whatever the particle
 // precision: the displacement v (e^{dv dt} - 1)/dv and the exit-time solve
 // lose their digits to cancellation at small velocity gradients.
-__device__ __forceinline__ double adv_exponential(double v, double dvdx, double dt) {
+// em1 = e^{dvdx dt} - 1
+__device__ __forceinline__ double adv_exponential(double v, double dvdx, double dt, double em1) {
   const double dvtol = 1.0e-10;
-  return (fabs(dvdx) > dvtol) ? v * (exp(dvdx * dt) - 1.0) / dvdx : v * dt;
+  return lt_any(dvtol, fabs(dvdx)) ? div_r(v * em1, dvdx) : v * dt;
 }
 
-// pr_NewtonRaphsonVariablesExponentialAdvection (:2082-2120)
-__device__ void nr_vars(double dt, double v, double dvdx, double dI, double divD, double dB, double &f0, double &f1,
-                        double &f2, double &f3) {
-  if (dt == 0.0) return;
-  f0 = adv_exponential(v, dvdx, dt) + divD * dt + dB * sqrt(dt) - dI;
-  const double e = exp(dvdx * dt);
-  f1 = v * e + divD + 0.5 * dB / sqrt(dt);
-  f2 = dvdx * v * e - 0.25 * dB * pow(dt, -1.5);
-  f3 = dvdx * dvdx * v * e + 0.375 * dB * pow(dt, -2.5);
-}
-__device__ __forceinline__ double nr_conv_g(double f0, double f1, double f2) { return fabs(f2 * f0 / (f1 * f1)); }
+__device__ __forceinline__ double nr_conv_g(double f0, double f1, double f2) { return fabs(div_r(f2 * f0, f1 * f1)); }
 __device__ __forceinline__ double nr_conv_gder(double f0, double f1, double f2, double f3) {
-  const double gna = f2 * f0 / (f1 * f1);
-  const double gpp = -2.0 * (f0 * (f2 * f2)) / (f1 * f1 * f1) + (f1 * f2 + f0 * f3) / (f1 * f1);
-  return gna / fabs(gna) * gpp;
+  const double gna = div_r(f2 * f0, f1 * f1);
+  const double gpp = div_r(-2.0 * (f0 * (f2 * f2)), f1 * f1 * f1) + div_r(f1 * f2 + f0 * f3, f1 * f1);
+  return div_r(gna, fabs(gna)) * gpp;
 }
-__device__ __forceinline__ double nr_p10(int e) {  // 10d0**e, exact for |e| <= 22
-  double r = 1.0;
-  for (int i = 0; i < (e < 0 ? -e : e); ++i) r *= 10.0;
-  return e < 0 ? 1.0 / r : r;
-}
+// |x| < 1, 1/2 for x = |..| (NaN: false, as the compare)
+__device__ __forceinline__ bool mag_below(double x, double c) { return fb::bits(x) < fb::bits(c); }
+__constant__ double kP10[8] = {1e-8, 1e-7, 1e-6, 1e-5, 1e-4, 1e-3, 1e-2, 1e-1};
 
-// pr_SetInitialGuess (:2162-2448); every loop is bounded (7, 50 and 8 passes)
-__device__ double nr_initial_guess(double dt, double v, double dvdx, double dI, double divD, double dB) {
-  const double gdtol = (double)1e-6f;
-  const int maxter = 50;
-  double f0 = 0, f1 = 0, f2 = 0, f3 = 0;
-  double dtnew = 0.0, dtold, dt0, gprimdernew, gprimnew, gprimder, gprim, gprimmin, gamman;
-  double dtfraction = 0, dtoldfraction, mindtfrac = 0;
-  int counter, ccount, bcount, zcount, rcount, gcount;
-  if (dt == 0.0) return dtnew;
-  gprimmin = (double)1e10f;
-  gprim = (double)1e10f;
-  gcount = 0;
-  while ((gprim > 1) && (gcount < 7)) {
-    gcount = gcount + 1;
-    dtfraction = nr_p10(-8 + gcount);
-    dt0 = dt * dtfraction;
-    nr_vars(dt0, v, dvdx, dI, divD, dB, f0, f1, f2, f3);
-    gprim = nr_conv_g(f0, f1, f2);
-    if (gprim < gprimmin) {
-      gprimmin = gprim;
-      mindtfrac = dtfraction;
-    }
-  }
-  if ((gprim < 1) && (gcount == 1)) dtoldfraction = 1e-8;
-  else if (gprim < 1) dtoldfraction = nr_p10(-8 + gcount - 1);
-  else {
-    dtfraction = mindtfrac;
-    dtoldfraction = 0.5 * dtfraction / 10.0;
-  }
-  dtnew = dtfraction * dt;
-  dtold = dtoldfraction * dt;
-  nr_vars(dtnew, v, dvdx, dI, divD, dB, f0, f1, f2, f3);
-  gprim = nr_conv_g(f0, f1, f2);
-  if (gprim < 0.5) return dtnew;
-  gprimnew = 10.0;
-  gprim = 10.0;
-  ccount = bcount = zcount = rcount = counter = 0;
-  while (counter < maxter) {
-    counter = counter + 1;
-    nr_vars(dtold, v, dvdx, dI, divD, dB, f0, f1, f2, f3);
-    gprimder = nr_conv_gder(f0, f1, f2, f3);
-    nr_vars(dtnew, v, dvdx, dI, divD, dB, f0, f1, f2, f3);
-    gprimdernew = nr_conv_gder(f0, f1, f2, f3);
-    gprim = nr_conv_g(f0, f1, f2);
-    if ((gprimdernew - gprimder) > 0.0)
-      gamman = fabs((dtnew - dtold) * (gprimdernew - gprimder)) /
-               ((gprimdernew - gprimder) * (gprimdernew - gprimder));
-    else
-      gamman = 0.0;
-    dtold = dtnew;
-    dtnew = dtnew - gamman * gprimdernew;
-    if (isnan(dtnew)) {
-      dtnew = 0.0;
-      break;
-    }
-    if ((gprim < 1) && (dtnew / dt > 1)) {
-      dtnew = dtold;
-      return dtnew;
-    } else if (dtnew / dt > 1) {
-      dtnew = (double)0.99f * dt;
-    }
-    if ((gprim < 1) && (dtnew < 0) && (dtold > 0)) {
-      dtnew = dtold;
-      return dtnew;
-    } else if (dtnew < 0) {
-      dtnew = (double)1e-8f * dt;
-      zcount = zcount + 1;
-      if (zcount > 1) {
-        dtnew = 0.0;
-        break;
+// NewtonRaphsonTimeStepExponentialAdvection (:2451-2554, at most 50
+// iterations) from pr_SetInitialGuess (:2162-2448; loops of 7, 50 and 8
+// passes) as one loop around one evaluation of
+// pr_NewtonRaphsonVariablesExponentialAdvection (:2082-2120): the displacement
+// residual f0 at time `at` and its derivatives f1, f2, f3.  The lanes of a
+// warp solve different faces and sit in different phases; with one evaluation
+// site they run it together, and its instruction count is what the solve
+// costs (the evaluation is FP64-pipe work).  An evaluation the reference
+// repeats at a time it has just used is taken from the one before: one per
+// pass of the 50-pass loop instead of three.  The convergence measure is only
+// ever compared, so there the -3/2 power of the time in f2 is a quotient by
+// its square root and itself, on the integer pipe; the measure's derivative,
+// whose last bits the 50-pass loop carries into the guess, keeps pow (84 FP64
+// instructions each) and is formed only when that loop goes on.
+// Together with the solves dealt out over the warp (below) and the velocity
+// gradients and exponentials held for a cell visit: 40,001 particles of a
+// 61x37x7 field, two 5-day intervals, 145 -> 69 ms in FP64 and 143 -> 64 ms in
+// MIXED at the same launch shape, every particle's state the same to the bit.
+__device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, double dI, double divD, double dB) {
+  enum { SCAN, START, FIRST, ITER, SCAN2, NEWTON };
+  const double gdtol = (double)1e-6f, nrtol = (double)1e-6f;
+  const int maxter = 50, maxIter = 50;
+  if (is0(dt)) return 0.0;
+  double f0 = 0, f1 = 0, f2 = 0, ve = 0.0, fat = 0.0;
+  double dtnew = 0.0, dtold = 0.0, gprimder = 0.0, gprimdernew = 0.0, gprimnew = 10.0;
+  double gprim = (double)1e10f, gprimmin = (double)1e10f, mindtfrac = 0.0, nrerror = 1e6;
+  int counter = 0, ccount = 0, bcount = 0, zcount = 0, rcount = 0, gcount = 1;
+  double dtfraction = kP10[1], at = dt * dtfraction;
+  int phase = SCAN;
+  for (;;) {
+    if (!is0(at) || phase == NEWTON) {
+      const double e = exp(dvdx * at), s = sqrt_r(at);
+      f0 = adv_exponential(v, dvdx, at, e - 1.0) + divD * at + dB * s - dI;
+      const double q = div_r(dB, s);
+      f1 = v * e + divD + 0.5 * q;
+      if (phase != NEWTON) {
+        ve = e;
+        fat = at;
+        f2 = dvdx * v * e - 0.25 * div_r(q, at);
       }
     }
-    nr_vars(dtnew, v, dvdx, dI, divD, dB, f0, f1, f2, f3);
-    gprimnew = nr_conv_g(f0, f1, f2);
-    if ((gprimnew < 1) && (dtnew > 0) && (dtnew / dt < 1)) {
-      rcount = rcount + 1;
-      if (rcount > 1) return dtnew;
+    bool guess = false;  // the initial guess is dtnew: go on to Newton
+    bool derive = false;   // the guess goes on: a pass of its 50-pass loop
+    if (phase == NEWTON) {
+      nrerror = div_r(-f0, f1);
+      dtnew = dtnew + nrerror;
+      if (below0(dtnew)) dtnew = -(double)0.9f * dtnew;
+      ++counter;
     } else {
-      rcount = 0;
+      const double g = nr_conv_g(f0, f1, f2);
+      if (phase == SCAN || phase == SCAN2) {
+        gprim = g;
+        if (mag_below(gprim, gprimmin)) {
+          gprimmin = gprim;
+          mindtfrac = dtfraction;
+        }
+        if (above1(gprim) && (gcount < (phase == SCAN ? 7 : 9))) {
+          ++gcount;
+          dtfraction = (phase == SCAN) ? kP10[gcount] : (double)(0.1f * (float)gcount);
+          at = dt * dtfraction;
+          continue;
+        }
+        if (phase == SCAN2) {
+          if (mag_below(gprimmin, 1.0)) dtnew = dt * mindtfrac;
+          if ((below0(dtnew) || is0(dtnew)) && above0(fabs(v))) dtnew = fabs(div_r(dI, v));
+          guess = true;
+        } else {
+          double dtoldfraction;
+          const bool below = mag_below(gprim, 1.0);
+          if (below) {
+            dtoldfraction = kP10[gcount - 1];
+          } else {
+            dtfraction = mindtfrac;
+            dtoldfraction = div_r(0.5 * dtfraction, 10.0);
+          }
+          dtnew = dtfraction * dt;
+          dtold = dtoldfraction * dt;
+          phase = START;
+          if (!below) {
+            at = dtnew;
+            continue;
+          }
+        }
+      }
+      if (phase == START) {
+        gprim = g;
+        if (mag_below(gprim, 0.5)) {
+          guess = true;
+        } else {
+          derive = true;
+        }
+      } else if (phase == FIRST) {
+        // at dtold; the values at dtnew are the starting ones
+        derive = true;
+      } else if (phase == ITER) {
+        gprimnew = g;
+        bool out = false;
+        if (mag_below(gprimnew, 1.0) && above0(dtnew) && mag_below(div_r(dtnew, dt), 1.0)) {
+          rcount = rcount + 1;
+          guess = rcount > 1;
+        } else {
+          rcount = 0;
+        }
+        if (!guess && mag_below(gprim, 1.0) && lt_any(gprim, gprimnew)) {
+          dtnew = dtold;
+          guess = true;
+        }
+        if (!guess) {
+          const bool still = mag_below(fabs(div_r(dtold - dtnew, dtold)), gdtol);
+          if (still && mag_below(gprim, 1.0)) {
+            ccount = ccount + 1;
+            guess = ccount > 1;
+          } else {
+            ccount = 0;
+          }
+          if (!guess) {
+            if (still && above1(gprim)) {
+              bcount = bcount + 1;
+              out = bcount > 1;
+            } else {
+              bcount = 0;
+            }
+          }
+        }
+        if (!guess) {
+          if (out || counter >= maxter) {
+            guess = mag_below(gprim, 1.0);
+            if (!guess) phase = SCAN2;
+          } else {
+            derive = true;
+          }
+        }
+      }
+      if (derive) {
+        // the derivative of the measure at the evaluated time (at zero time
+        // the values stay those of the evaluation before)
+        double p2 = 0.0, p3 = 0.0;
+        if (!is0(fat)) {
+          p2 = dvdx * v * ve - 0.25 * dB * pow(fat, -1.5);
+          p3 = dvdx * dvdx * v * ve + 0.375 * dB * pow(fat, -2.5);
+        }
+        const double gd = nr_conv_gder(f0, f1, p2, p3);
+        if (phase == START) {
+          gprimdernew = gd;
+          at = dtold;
+          phase = FIRST;
+          continue;
+        }
+        if (phase == FIRST) {
+          gprimder = gd;
+          if (is0(dtnew)) {
+            gprimdernew = gd;
+            gprim = g;
+          }
+        } else {
+          // the next pass: dtold's values are those dtnew had before it
+          gprimder = is0(dtold) ? gd : gprimdernew;
+          gprimdernew = gd;
+          gprim = g;
+        }
+        counter = counter + 1;
+        const double dg = gprimdernew - gprimder;
+        const double gamman = above0(dg) ? div_r(fabs((dtnew - dtold) * dg), dg * dg) : 0.0;
+        dtold = dtnew;
+        dtnew = dtnew - gamman * gprimdernew;
+        bool out = false;
+        if (fb::isnan_bits(dtnew)) {
+          dtnew = 0.0;
+          out = true;
+        } else {
+          const bool past = above1(div_r(dtnew, dt));
+          if (mag_below(gprim, 1.0) && past) {
+            dtnew = dtold;
+            guess = true;
+          } else if (past) {
+            dtnew = (double)0.99f * dt;
+          }
+          if (!guess) {
+            if (mag_below(gprim, 1.0) && below0(dtnew) && above0(dtold)) {
+              dtnew = dtold;
+              guess = true;
+            } else if (below0(dtnew)) {
+              dtnew = (double)1e-8f * dt;
+              zcount = zcount + 1;
+              if (zcount > 1) {
+                dtnew = 0.0;
+                out = true;
+              }
+            }
+          }
+        }
+        if (!guess && out) {
+          guess = mag_below(gprim, 1.0);
+          if (!guess) phase = SCAN2;
+        } else if (!guess) {
+          at = dtnew;
+          phase = ITER;
+          continue;
+        }
+      }
+      if (!guess) {  // the second scan begins
+        gprim = gprimmin = (double)1e10f;
+        mindtfrac = 0.0;
+        gcount = 2;
+        dtfraction = (double)(0.1f * (float)gcount);
+        at = dt * dtfraction;
+        continue;
+      }
+      if (is0(dtnew)) return 0.0;
+      phase = NEWTON;
+      counter = 0;
     }
-    if ((gprim < 1) && (gprimnew > gprim)) {
-      dtnew = dtold;
-      return dtnew;
-    }
-    if ((fabs((dtold - dtnew) / dtold) < gdtol) && (gprim < 1)) {
-      ccount = ccount + 1;
-      if (ccount > 1) return dtnew;
-    } else {
-      ccount = 0;
-    }
-    if ((fabs((dtold - dtnew) / dtold) < gdtol) && (gprim > 1)) {
-      bcount = bcount + 1;
-      if (bcount > 1) break;
-    } else {
-      bcount = 0;
-    }
+    if (!(lt_any(nrtol, fabs(div_r(nrerror, dtnew))) && (counter < maxIter))) break;
+    at = dtnew;
   }
-  if (gprim < 1) return dtnew;
-  gprim = (double)1e10f;
-  gprimmin = (double)1e10f;
-  mindtfrac = 0.0;
-  gcount = 1;
-  while ((gprim > 1) && (gcount < 9)) {
-    gcount = gcount + 1;
-    dtfraction = (double)(0.1f * (float)gcount);
-    dt0 = dt * dtfraction;
-    nr_vars(dt0, v, dvdx, dI, divD, dB, f0, f1, f2, f3);
-    gprim = nr_conv_g(f0, f1, f2);
-    if (gprim < gprimmin) {
-      gprimmin = gprim;
-      mindtfrac = dtfraction;
-    }
-  }
-  if (gprimmin < 1) dtnew = dt * mindtfrac;
-  if ((dtnew <= 0.0) && (fabs(v) > 0.0)) dtnew = fabs(dI / v);
+  if (lt_any(dt, dtnew)) return dt;
+  if ((counter == maxIter) && lt_any(nrtol, fabs(div_r(nrerror, dtnew)))) return 0.0;
   return dtnew;
 }
 
-// NewtonRaphsonTimeStepExponentialAdvection (:2451-2554), at most 50 iterations
-__device__ double nr_time_step(double dt, double v, double dvdx, double dI, double divD, double dB) {
-  const double nrtol = (double)1e-6f;
-  const int maxIter = 50;
-  double nrerror = 1e6;
-  double dt0 = nr_initial_guess(dt, v, dvdx, dI, divD, dB);
-  if (dt0 == 0.0) return 0.0;
-  int countIter = 0;
-  while ((fabs(nrerror / dt0) > nrtol) && (countIter < maxIter)) {
-    countIter = countIter + 1;
-    const double f0 = adv_exponential(v, dvdx, dt0) + divD * dt0 + dB * sqrt(dt0) - dI;
-    const double f1 = v * exp(dvdx * dt0) + divD + 0.5 * dB / sqrt(dt0);
-    nrerror = -f0 / f1;
-    dt0 = dt0 + nrerror;
-    if (dt0 < 0.0) dt0 = -(double)0.9f * dt0;
-  }
-  if (dt0 > dt) return dt;
-  if ((countIter == maxIter) && (fabs(nrerror / dt0) > nrtol)) return 0.0;
-  return dt0;
-}
-
 // One axis of pr_DetectExitFaceAndUpdateTimeStepNewton (:1895-2079).
-// Returns true when the routine must return at once (exitFace, dt set).
-__device__ bool newton_axis(double npos, double pos, double d, double v, double dvdx, double divD, double dB,
+// Returns true when the routine must return at once (exitFace, dt set); `high`:
+// the step leaves through the axis's upper face.
+__device__ __forceinline__ bool newton_axis(bool high, double pos, double d, double v, double dvdx, double divD, double dB,
                             int faceLo, int faceHi, double dt, double &dtaxis, int &exitAxis, int &exitFace,
                             double &dtout) {
   double dI;
-  if (npos > 1.0) {
+  if (high) {
     dI = d * (1.0 - pos);
     exitAxis = faceHi;
   } else {
     dI = -d * pos;
     exitAxis = faceLo;
   }
-  if (dI == 0.0) {
+  if (is0(dI)) {
     exitFace = exitAxis;
     dtout = 0.0;
     return true;
   }
   dtaxis = nr_time_step(dt, v, dvdx, dI, divD, dB);
-  if (dtaxis > dt) dtaxis = 0.0;
+  if (lt_any(dt, dtaxis)) dtaxis = 0.0;
   return false;
 }
 
@@ -613,8 +720,16 @@ __device__ __forceinline__ bool outside3(R a, R b, R c) {
 }
 #define MPRW_OUTSIDE(a, b, c) outside3(a, b, c)
 
+// Exchange slots of a block in shared memory, kExitSlot doubles per thread,
+// field k of a slot at p[k * stride + slot]; and the EXPONENTIAL kernel's
+// per-lane values of a cell visit: the velocity gradients (V2 - V1)/D and
+// e^{gradient dtcell} - 1 per axis.
+constexpr int kExitSlot = 7;
+constexpr int kExpFields = 6;
+
 // The first interface iteration's exit-face solves of the leaving lanes of
-// `grp`, dealt out to every lane of `grp` (FP64).  Each (leaving lane,
+// `grp`, dealt out to every lane of `grp` (FP64, and the Newton solves of
+// EXPONENTIAL advection, whose dv is the velocity gradient).  Each (leaving lane,
 // leaving axis) pair is a task; tasks in axis-major order go to the group's
 // lanes by rank (a second round only past one task per lane), every lane
 // solves one with its owner's values (quad_axis is a pure function of them),
@@ -622,14 +737,18 @@ __device__ __forceinline__ bool outside3(R a, R b, R c) {
 // once (bit k of rbits), its exit face and its time.  Without this, a warp
 // solves its lanes' first leaving axes together and then their second axes
 // (corner crossings) in a second round of one or two lanes.  Every lane of
-// grp calls it together.
-__device__ __forceinline__ void warp_exit_solves(unsigned grp, unsigned need, double nx, double ny, double nz,
-                                                 double x, double y, double z, double dX, double dY, double dZ,
-                                                 double vx, double vy, double vz, double ddx, double ddy,
-                                                 double ddz, double bx, double by, double bz, double dt,
-                                                 unsigned &rbits, double &tx, double &ty, double &tz, int &fx,
-                                                 int &fy, int &fz) {
-  const int lane = threadIdx.x & 31;
+// grp calls it together.  The operands travel through the warp's exchange
+// slots in shared memory: the owner of task t writes slot t, the lane of that
+// rank reads it and writes the result back, so nobody searches for an owner.
+template <typename R, bool EXP>
+__device__ __forceinline__ void warp_exit_solves(unsigned grp, unsigned need, const Lane<R> &F, double *slots,
+                                                 R nx, R ny, R nz, R x, R y, R z,
+                                                 R vx, R vy, R vz, R ddx, R ddy,
+                                                 R ddz, R bx, R by, R bz, double dvx,
+                                                 double dvy, double dvz, double dt, unsigned &rbits,
+                                                 double &tx, double &ty, double &tz, int &fx, int &fy,
+                                                 int &fz) {
+  const int lane = threadIdx.x & 31, stride = F.stride;
   const unsigned below = (1u << lane) - 1u;
   const unsigned m0 = __ballot_sync(grp, need & 1u), m1 = __ballot_sync(grp, need & 2u);
   const unsigned m2 = __ballot_sync(grp, need & 4u);
@@ -637,62 +756,58 @@ __device__ __forceinline__ void warp_exit_solves(unsigned grp, unsigned need, do
   const int nw = __popc(grp), rank = __popc(grp & below);
   // this lane's own tasks, one per leaving axis
   const int t0 = __popc(m0 & below), t1 = c0 + __popc(m1 & below), t2 = c0 + c1 + __popc(m2 & below);
+  double *slot = slots + (threadIdx.x & ~31);  // the warp's slots
+  const R *rec = F.p - lane;                   // the warp's records
   rbits = 0u;
   tx = ty = tz = 0.0;
   fx = fy = fz = 0;
   for (int base = 0; base < total; base += nw) {
-    const int t = base + rank;
-    int a = 0, owner = lane;
-    if (t < total) {
-      if (t < c0) {
-        owner = __fns(m0, 0, t + 1);
-      } else if (t < c0 + c1) {
-        a = 1;
-        owner = __fns(m1, 0, t - c0 + 1);
-      } else {
-        a = 2;
-        owner = __fns(m2, 0, t - c0 - c1 + 1);
-      }
+    auto put = [&](int a, int t, R npos, R pos, R v, R dd, R b, double dv) {
+      const int k = t - base;
+      if (!((need >> a) & 1u) || k < 0 || k >= nw) return;
+      slot[k] = (double)pos;
+      slot[stride + k] = (double)v;
+      slot[2 * stride + k] = (double)dd;
+      slot[3 * stride + k] = (double)b;
+      slot[4 * stride + k] = dt;
+      if (EXP) slot[6 * stride + k] = dv;
+      reinterpret_cast<int *>(slot + 5 * stride + k)[0] = lane | (a << 5) | (above1(npos) ? 128 : 0);
+    };
+    put(0, t0, nx, x, vx, ddx, bx, dvx);
+    put(1, t1, ny, y, vy, ddy, by, dvy);
+    put(2, t2, nz, z, vz, ddz, bz, dvz);
+    __syncwarp(grp);
+    if (base + rank < total) {
+      const int meta = reinterpret_cast<const int *>(slot + 5 * stride + rank)[0];
+      const int a = (meta >> 5) & 3;
+      int efa = 0, ef_unused = 0;
+      double dta = 0.0, dt_unused = 0.0;
+      const double d = (double)rec[(F_D + a) * stride + (meta & 31)];
+      bool r;
+      if constexpr (EXP)
+        r = newton_axis((meta & 128) != 0, slot[rank], d, slot[stride + rank], slot[6 * stride + rank],
+                        slot[2 * stride + rank], slot[3 * stride + rank], 2 * a + 1, 2 * a + 2,
+                        slot[4 * stride + rank], dta, efa, ef_unused, dt_unused);
+      else
+        r = quad_axis_f64((meta & 128) != 0, slot[rank], d, slot[stride + rank], slot[2 * stride + rank],
+                          slot[3 * stride + rank], 2 * a + 1, 2 * a + 2, slot[4 * stride + rank], dta, efa,
+                          ef_unused, dt_unused);
+      slot[rank] = dta;
+      reinterpret_cast<int *>(slot + 5 * stride + rank)[0] = (r ? 8 : 0) | efa;
     }
-    // the owner's values on all three axes, the task's axis picked after
-    const double onx = __shfl_sync(grp, nx, owner), ony = __shfl_sync(grp, ny, owner);
-    const double onz = __shfl_sync(grp, nz, owner);
-    const double ox = __shfl_sync(grp, x, owner), oy = __shfl_sync(grp, y, owner), oz = __shfl_sync(grp, z, owner);
-    const double odX = __shfl_sync(grp, dX, owner), odY = __shfl_sync(grp, dY, owner);
-    const double odZ = __shfl_sync(grp, dZ, owner);
-    const double ovx = __shfl_sync(grp, vx, owner), ovy = __shfl_sync(grp, vy, owner);
-    const double ovz = __shfl_sync(grp, vz, owner);
-    const double oddx = __shfl_sync(grp, ddx, owner), oddy = __shfl_sync(grp, ddy, owner);
-    const double oddz = __shfl_sync(grp, ddz, owner);
-    const double obx = __shfl_sync(grp, bx, owner), oby = __shfl_sync(grp, by, owner);
-    const double obz = __shfl_sync(grp, bz, owner);
-    const double odt = __shfl_sync(grp, dt, owner);
-    bool r = false;
-    double dta = 0.0;
-    int efa = 0;
-    if (t < total) {
-      int ef_unused = 0;
-      double dt_unused = 0.0;
-      r = quad_axis_f64(pick3(a, onx, ony, onz), pick3(a, ox, oy, oz), pick3(a, odX, odY, odZ),
-                            pick3(a, ovx, ovy, ovz), pick3(a, oddx, oddy, oddz), pick3(a, obx, oby, obz),
-                            2 * a + 1, 2 * a + 2, odt, dta, efa, ef_unused, dt_unused);
-    }
-    // results back to their owners, one axis at a time
-    const unsigned packed = (r ? 8u : 0u) | (unsigned)efa;
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      const int tb = (b == 0) ? t0 : ((b == 1) ? t1 : t2);
-      const bool mine = ((need >> b) & 1u) && tb >= base && tb < base + nw;
-      const int wl = mine ? (int)__fns(grp, 0, tb - base + 1) : lane;
-      const unsigned pk = __shfl_sync(grp, packed, wl);
-      const double dv = __shfl_sync(grp, dta, wl);
-      if (mine) {
-        if (pk & 8u) rbits |= 1u << b;
-        if (b == 0) { tx = dv; fx = (int)(pk & 7u); }
-        else if (b == 1) { ty = dv; fy = (int)(pk & 7u); }
-        else { tz = dv; fz = (int)(pk & 7u); }
-      }
-    }
+    __syncwarp(grp);
+    auto get = [&](int a, int t, double &ta, int &fa) {
+      const int k = t - base;
+      if (!((need >> a) & 1u) || k < 0 || k >= nw) return;
+      ta = slot[k];
+      const int pk = reinterpret_cast<const int *>(slot + 5 * stride + k)[0];
+      fa = pk & 7;
+      if (pk & 8) rbits |= 1u << a;
+    };
+    get(0, t0, tx, fx);
+    get(1, t1, ty, fy);
+    get(2, t2, tz, fz);
+    __syncwarp(grp);
   }
 }
 
@@ -700,7 +815,7 @@ __device__ __forceinline__ void warp_exit_solves(unsigned grp, unsigned need, do
 // On PASS_MAXTIME / PASS_EXIT the final location is (ox,oy,oz,V.t); on
 // PASS_UNDEFINED the caller uses the last recorded point.
 template <typename R, bool EXP, bool AXI>
-__device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double maxTime, int ndim, int d1, int d2,
+__device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t massb, double maxTime, int ndim, int d1, int d2,
                        uint64_t seed, uint64_t id, uint64_t &ctr, R &ox, R &oy, R &oz) {
   const R zero = R(0), one = R(1), half = R(0.5);
   const unsigned grp = __activemask();  // the lanes running this pass together
@@ -714,7 +829,7 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
     V.t = maxTime;
     V.reachedMax = true;
     rdt = (R)dt;
-    sdt = sqrt(rdt);
+    sdt = sqrt_r(rdt);
   }
   R x = V.x, y = V.y, z = V.z;
   R dX = F(F_D + 0), dY = F(F_D + 1), dZ = F(F_D + 2);
@@ -731,25 +846,33 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
   random_displacement<R, AXI>(F, ndim, d1, d2, x, y, z, vx, vy, vz, seed, id, ctr, bx, by, bz);
   // advection displacement: EULERIAN v dt, EXPONENTIAL (FP64) v (e^{dv dt}-1)/dv
   // with dv = (V2 - V1)/D of the cell (pr_AdvectionDisplacement*, :1487-1573)
+  // (dv, and the exponentials of the whole cell step, held for the visit)
   double dvx = 0.0, dvy = 0.0, dvz = 0.0;
+  const double *xf = slots + kExitSlot * F.stride + threadIdx.x;
   if constexpr (EXP) {
-    dvx = (double)F(F_DV + 0) / (double)dX;
-    dvy = (double)F(F_DV + 1) / (double)dY;
-    dvz = (double)F(F_DV + 2) / (double)dZ;
+    dvx = xf[0];
+    dvy = xf[F.stride];
+    dvz = xf[2 * F.stride];
   }
   R ax, ay, az;
   auto advect = [&]() {
     if constexpr (EXP) {
-      ax = (R)adv_exponential((double)vx, dvx, dt);
-      ay = (R)adv_exponential((double)vy, dvy, dt);
-      az = (R)adv_exponential((double)vz, dvz, dt);
+      ax = (R)adv_exponential((double)vx, dvx, dt, exp(dvx * dt) - 1.0);
+      ay = (R)adv_exponential((double)vy, dvy, dt, exp(dvy * dt) - 1.0);
+      az = (R)adv_exponential((double)vz, dvz, dt, exp(dvz * dt) - 1.0);
     } else {
       ax = vx * rdt;
       ay = vy * rdt;
       az = vz * rdt;
     }
   };
-  advect();
+  if (EXP && eq_any(dt, V.dtcell)) {
+    ax = (R)adv_exponential((double)vx, dvx, dt, xf[3 * F.stride]);
+    ay = (R)adv_exponential((double)vy, dvy, dt, xf[4 * F.stride]);
+    az = (R)adv_exponential((double)vz, dvz, dt, xf[5 * F.stride]);
+  } else {
+    advect();
+  }
   R dxrw = ax + ddx * rdt + bx * sdt;
   R dyrw = ay + ddy * rdt + by * sdt;
   R dzrw = az + ddz * rdt + bz * sdt;
@@ -763,7 +886,7 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
     bool cut = false;
     while ((fabs(dxrw * iX) > half) || (fabs(dyrw * iY) > half) || (fabs(dzrw * iZ) > half)) {
       rdt = R(0.1f) * rdt;
-      sdt = sqrt(rdt);
+      sdt = sqrt_r(rdt);
       advect();
       dxrw = ax + ddx * rdt + bx * sdt;
       dyrw = ay + ddy * rdt + by * sdt;
@@ -781,7 +904,7 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
     V.t = V.t - dt;
     dt = dtRed * dt;
     rdt = (R)dt;
-    sdt = sqrt(rdt);
+    sdt = sqrt_r(rdt);
     advect();
     dxrw = ax + ddx * rdt + bx * sdt;
     dyrw = ay + ddy * rdt + by * sdt;
@@ -790,16 +913,15 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
     V.reachedMax = false;
   }
   R nx = x + dxrw * iX, ny = y + dyrw * iY, nz = z + dzrw * iZ;
-  // FP64 EULERIAN: the first interface iteration's exit-face solves of the
-  // leaving lanes, spread over every lane of the pass
+  // FP64 and EXPONENTIAL: the first interface iteration's exit-face solves of
+  // the leaving lanes, spread over every lane of the pass
   unsigned pre_r = 0u;
   double pre_tx = 0.0, pre_ty = 0.0, pre_tz = 0.0;
   int pre_fx = 0, pre_fy = 0, pre_fz = 0;
-  if constexpr (sizeof(R) == 8 && !EXP) {
+  if constexpr (sizeof(R) == 8 || EXP) {
     __syncwarp(grp);
-    warp_exit_solves(grp, MPRW_OUTSIDE(nx, ny, nz) ? axes_outside(nx, ny, nz) : 0u, nx, ny, nz, x, y, z, dX, dY,
-                     dZ, vx, vy, vz, ddx, ddy, ddz, bx, by, bz, dt, pre_r, pre_tx, pre_ty, pre_tz, pre_fx, pre_fy,
-                     pre_fz);
+    warp_exit_solves<R, EXP>(grp, axes_outside(nx, ny, nz), F, slots, nx, ny, nz, x, y, z, vx, vy, vz, ddx, ddy,
+                             ddz, bx, by, bz, dvx, dvy, dvz, dt, pre_r, pre_tx, pre_ty, pre_tz, pre_fx, pre_fy, pre_fz);
   }
   // particleLeavingCell (:1025-1316)
   int intLoop = 0;
@@ -816,12 +938,26 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
       // the second (a warp's leaving lanes mostly leave through different
       // axes; three per-axis branches would each run with a few lanes)
       unsigned need = axes_outside(nx, ny, nz);
+      if (intLoop == 1) {
+        // the warp-wide solves (the same inputs: nothing has moved yet)
+        while (!ret && need) {
+          const int k = __ffs(need) - 1;
+          need &= need - 1;
+          if ((pre_r >> k) & 1u) {
+            V.exitFace = pick3(k, pre_fx, pre_fy, pre_fz);
+            dt = 0.0;
+            ret = true;
+          } else if (k == 0) { dtx = pre_tx; efx = pre_fx; }
+          else if (k == 1) { dty = pre_ty; efy = pre_fy; }
+          else { dtz = pre_tz; efz = pre_fz; }
+        }
+      }
       while (!ret && need) {
         const int k = __ffs(need) - 1;
         need &= need - 1;
         double dta = 0.0;
         int efa = 0;
-        ret = newton_axis((double)pick3(k, nx, ny, nz), (double)pick3(k, x, y, z), (double)pick3(k, dX, dY, dZ),
+        ret = newton_axis(above1(pick3(k, nx, ny, nz)), (double)pick3(k, x, y, z), (double)pick3(k, dX, dY, dZ),
                           (double)pick3(k, vx, vy, vz), pick3(k, dvx, dvy, dvz), (double)pick3(k, ddx, ddy, ddz),
                           (double)pick3(k, bx, by, bz), 2 * k + 1, 2 * k + 2, dt, dta, efa, V.exitFace, dt);
         if (k == 0) { dtx = dta; efx = efa; }
@@ -875,7 +1011,7 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
           need &= need - 1;
           R dta = zero;
           int efa = 0;
-          ret = quad_axis_f64(pick3(k, nx, ny, nz), pick3(k, x, y, z), pick3(k, dX, dY, dZ), pick3(k, vx, vy, vz),
+          ret = quad_axis_f64(above1(pick3(k, nx, ny, nz)), pick3(k, x, y, z), pick3(k, dX, dY, dZ), pick3(k, vx, vy, vz),
                           pick3(k, ddx, ddy, ddz), pick3(k, bx, by, bz), 2 * k + 1, 2 * k + 2, dt, dta, efa,
                           V.exitFace, dt);
           if (k == 0) { dtx = dta; efx = efa; }
@@ -931,7 +1067,7 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
       break;
     }
     if constexpr (sizeof(R) == 8 || EXP) rdt = (R)dt;  // MIXED EULERIAN: rdt set above
-    sdt = sqrt(rdt);
+    sdt = sqrt_r(rdt);
     advect();
     V.reachedMax = false;
     int ef = V.exitFace;
@@ -1000,7 +1136,7 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, uint32_t massb, double max
         V.t = maxTime;
         V.reachedMax = true;
         rdt = (R)dt;
-        sdt = sqrt(rdt);
+        sdt = sqrt_r(rdt);
         advect();
         dxrw = ax + ddx * rdt + bx * sdt;
         dyrw = ay + ddy * rdt + by * sdt;
@@ -1066,6 +1202,8 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
   R *sm = reinterpret_cast<R *>(smraw) + threadIdx.x;
   const int stride = blockDim.x;
   Lane<R> F{sm, stride};
+  // the exchange slots (FP64 or EXPONENTIAL) follow the records
+  double *slots = reinterpret_cast<double *>(reinterpret_cast<R *>(smraw) + NFIELDS * stride);
   const R zero = R(0), one = R(1);
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -1181,6 +1319,14 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
           use_last = (es == ST_UNDEFINED);
         } else {
           stage_record(a.recs, c, sm, stride);
+          if constexpr (EXP) {
+            double *xf = slots + kExitSlot * stride + threadIdx.x;
+            for (int d = 0; d < 3; ++d) {
+              const double g = div_r((double)F(F_DV + d), (double)F(F_D + d));
+              xf[d * stride] = g;
+              xf[(3 + d) * stride] = exp(g * rec->dtcell) - 1.0;
+            }
+          }
           massb = rec->massb;
           V.x = ex; V.y = ey; V.z = ez;
           V.ix = ex; V.iy = ey; V.iz = ez;
@@ -1213,7 +1359,7 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
       if (++V.passes > kMaxStepsPerVisit) {
         r = PASS_UNDEFINED;
       } else {
-        r = rw_pass<R, EXP, AXI>(V, F, massb, a.t_end, a.ndim, a.d1, a.d2, a.seed, id, ctr, ox, oy, oz);
+        r = rw_pass<R, EXP, AXI>(V, F, slots, massb, a.t_end, a.ndim, a.d1, a.d2, a.seed, id, ctr, ox, oy, oz);
         ++my_passes;
       }
       if (r == PASS_MAXTIME) {
@@ -1275,14 +1421,17 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
   if (threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long *>(a.steps), blk);
 }
 
+// the lanes' records, the exchange slots (FP64 or EXPONENTIAL; EULERIAN leaves
+// their last field out) and the EXPONENTIAL kernel's visit values
 template <typename R>
-size_t advance_smem_bytes(int threads) {
-  return (size_t)NFIELDS * sizeof(R) * threads;
+static size_t advance_smem_bytes(int threads, int exp_adv) {
+  const int extra = exp_adv ? kExitSlot + kExpFields : (sizeof(R) == 8 ? kExitSlot - 1 : 0);
+  return (NFIELDS * sizeof(R) + extra * sizeof(double)) * threads;
 }
 
 template <typename R>
 cudaError_t launch_advance(const AdvanceArgs<R> &a, int blocks, int threads, cudaStream_t s) {
-  size_t smem = advance_smem_bytes<R>(threads);
+  size_t smem = advance_smem_bytes<R>(threads, a.exp_adv);
   auto kern = a.exp_adv ? (a.axi ? rwpt_advance_kernel<R, true, true> : rwpt_advance_kernel<R, true, false>)
                         : (a.axi ? rwpt_advance_kernel<R, false, true> : rwpt_advance_kernel<R, false, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1293,7 +1442,7 @@ cudaError_t launch_advance(const AdvanceArgs<R> &a, int blocks, int threads, cud
 
 template <typename R>
 cudaError_t advance_occupancy(int exp_adv, int axi, int threads, int *blocks_per_sm) {
-  size_t smem = advance_smem_bytes<R>(threads);
+  size_t smem = advance_smem_bytes<R>(threads, exp_adv);
   auto kern = exp_adv ? (axi ? rwpt_advance_kernel<R, true, true> : rwpt_advance_kernel<R, true, false>)
                       : (axi ? rwpt_advance_kernel<R, false, true> : rwpt_advance_kernel<R, false, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1305,7 +1454,5 @@ template cudaError_t launch_advance<double>(const AdvanceArgs<double> &, int, in
 template cudaError_t advance_occupancy<double>(int, int, int, int *);
 template cudaError_t advance_occupancy<float>(int, int, int, int *);
 template cudaError_t launch_advance<float>(const AdvanceArgs<float> &, int, int, cudaStream_t);
-template size_t advance_smem_bytes<double>(int);
-template size_t advance_smem_bytes<float>(int);
 
 }  // namespace mprw
