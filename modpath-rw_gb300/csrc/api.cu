@@ -771,9 +771,62 @@ int max_blocks_per_sm(mprw_handle *h) {
   return nb;
 }
 
+// EXPONENTIAL: particles from which every resident warp is filled
+constexpr int64_t kExpSpread = 150000;
+
 int default_blocks_per_sm(mprw_handle *h) {
   // EULERIAN MIXED is compiled for 3 resident blocks per SM (80 registers)
   return (h->opt.precision == MPRW_MIXED && h->opt.advection_kind != 1) ? 3 : 1;
+}
+
+// Launch shape of the step kernel for h->n particles at up to bps resident
+// blocks of step_threads() per SM.
+struct StepShape {
+  int threads, lanes;  // threads per block; lanes of each warp that take particles
+  int64_t blocks;
+};
+
+// Many particles fill every resident warp.  With fewer, the kernel ends with
+// its longest particle, and a particle's pass takes the longer the more warps
+// share its SM's FP64 pipe (FP64, EXPONENTIAL: a pass holds that pipe for some
+// 200 warp instructions of 16 clocks) and the more lanes of its warp branch
+// (exits, the jump limiter, Newton): so they are spread over all SMs, few
+// warps per SM first (four, one per scheduler; eight in MIXED, bound by
+// latency), then few lanes per warp, two at least.  Measured, two intervals
+// (ms, all warps full -> spread): FP64 column of 2,000 particles 2.39 -> 1.15,
+// 30,000: 2.55 -> 1.80; FP64 100x60x10 field, 4,000: 8.35 -> 5.77, 16,000: 9.29
+// -> 7.0; MIXED, 4,000: 3.23 -> 1.97; EXPONENTIAL, 4,000: 39 -> 18, 40,000: 52 ->
+// 41 (150,000: equal).  Past one particle per lane the FP64 warps are levelled
+// over the rounds (100,000 particles, 12 warps -> 11: 7.07 -> 6.71); MIXED runs
+// blocks of four warps (1,000,000: equal; 40,000 in the column: 0.78 -> 0.70).
+StepShape step_shape(mprw_handle *h, int bps) {
+  const bool mixed = h->opt.precision == MPRW_MIXED, exp_adv = h->opt.advection_kind == 1;
+  const int64_t sms = h->sms;
+  const int max_warps = step_threads(!mixed, exp_adv) / 32 * bps;  // per SM
+  const int64_t per = (h->n + sms - 1) / sms;                      // particles per SM
+  auto ceil_div = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+  int64_t warps, lanes = 32;  // warps per SM
+  if (exp_adv) {
+    // Newton's passes differ most between particles: 0.6 lanes per particle
+    warps = h->n < kExpSpread ? 4 : max_warps;
+    if (h->n < kExpSpread) lanes = ceil_div(6 * per, 40);
+  } else if (mixed) {
+    warps = per <= 256 ? 8 : max_warps;
+    lanes = ceil_div(per, 8);
+  } else {
+    const int64_t rounds = ceil_div(per, 32 * max_warps);
+    warps = per <= 128 ? std::min<int64_t>(4, ceil_div(per, 2)) : ceil_div(per, 32 * rounds);
+    lanes = ceil_div(per, warps);
+  }
+  warps = std::max<int64_t>(1, std::min<int64_t>(warps, max_warps));
+  lanes = std::max<int64_t>(2, std::min<int64_t>(lanes, 32));
+  StepShape r;
+  r.lanes = (int)lanes;
+  // FP64: one block per SM of all its warps; the others: blocks of four warps
+  const int wpb = (mixed || exp_adv) ? (int)std::min<int64_t>(4, warps) : (int)warps;
+  r.threads = 32 * wpb;
+  r.blocks = std::min<int64_t>(sms * std::max<int64_t>(1, warps / wpb), ceil_div(h->n, lanes * wpb));
+  return r;
 }
 
 // One launch of the persistent step kernel over every particle, processing
@@ -781,10 +834,9 @@ int default_blocks_per_sm(mprw_handle *h) {
 int launch_step(mprw_handle *h, double t_begin, double t_end, int bps, bool use_perm, float *ms, int64_t *steps) {
   cudaStream_t s = h->stream;
   CK(cudaMemsetAsync(h->d_counters, 0, 4 * sizeof(unsigned long long), s));
-  const int threads = step_threads(h->opt.precision != MPRW_MIXED, h->opt.advection_kind == 1);
-  int64_t need = (h->n + threads - 1) / threads;
-  int64_t blocks = (int64_t)h->sms * bps;
-  if (need < blocks) blocks = need;
+  const StepShape shape = step_shape(h, bps);
+  const int threads = shape.threads, lanes = shape.lanes;
+  const int64_t blocks = shape.blocks;
   CK(cudaEventRecord(h->ev0, s));
   if (h->opt.precision == MPRW_MIXED) {
     AdvanceArgs<float> a{};
@@ -812,6 +864,7 @@ int launch_step(mprw_handle *h, double t_begin, double t_end, int bps, bool use_
     a.seed = h->opt.rng_seed;
     a.exp_adv = h->opt.advection_kind == 1;
     a.axi = h->opt.dispersion_model == 1;
+    a.lanes = lanes;
     CK(launch_advance<float>(a, (int)blocks, threads, s));
   } else {
     AdvanceArgs<double> a{};
@@ -839,6 +892,7 @@ int launch_step(mprw_handle *h, double t_begin, double t_end, int bps, bool use_
     a.seed = h->opt.rng_seed;
     a.exp_adv = h->opt.advection_kind == 1;
     a.axi = h->opt.dispersion_model == 1;
+    a.lanes = lanes;
     CK(launch_advance<double>(a, (int)blocks, threads, s));
   }
   h->launches += 1;

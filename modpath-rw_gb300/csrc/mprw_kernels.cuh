@@ -32,6 +32,7 @@ struct AdvanceArgs {
   uint64_t seed;
   int exp_adv;  // EXPONENTIAL advection with the Newton exit time (else EULERIAN)
   int axi;      // linear axisymmetric dispersion (else linear isotropic)
+  int lanes;    // lanes of each warp that take particles (32 but for few particles)
 };
 
 template <typename R>

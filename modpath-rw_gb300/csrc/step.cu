@@ -1210,7 +1210,7 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
 
   int64_t my_passes = 0;
   int64_t p = -1;        // particle being tracked (index into the state arrays)
-  bool open = true;      // the queue may still have particles for this lane
+  bool open = lane < a.lanes;  // the queue may still have particles for this lane
   int32_t c = 0;         // current cell (0-based)
   bool need_cell = false;
   uint64_t id = 0, ctr = 0;
