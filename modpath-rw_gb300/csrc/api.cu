@@ -1251,15 +1251,7 @@ int histogram_device(mprw_handle *h, const double origin[3], const double bin_si
     nb_out = (int64_t)h->h_counters[2];
     eff = 1.0;  // unit weights: Kish nEffective = totalMass, effective mass 1
   } else {
-    size_t arr = ((size_t)n * 8 + 255) / 256 * 256;
-    void *tmp = nullptr;
-    CK(cudaMalloc(&tmp, arr));
-    int64_t *bin_of = (int64_t *)tmp;
-    a.bin_of = bin_of;
-    cudaError_t e = launch_hist_bins(a, s);
-    if (e == cudaSuccess)
-      e = ordered_bin_sums(bin_of, h->d_mass, h->d_status, n, nbins, h->d_counts, &total, &sw2, &h->scratch,
-                           &h->scratch_bytes, s);
+    cudaError_t e = ordered_bin_sums(a, h->d_mass, nbins, h->d_counts, &total, &sw2, &h->scratch, &h->scratch_bytes, s);
     if (e == cudaSuccess && total != 0.0) {
       double neff = total * total / sw2;  // Kish (Histogram.F90:338-340)
       eff = total / neff;
@@ -1269,7 +1261,6 @@ int histogram_device(mprw_handle *h, const double origin[3], const double bin_si
       }
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(tmp);
     CK(e);
     h->launches += 5;
     nb_out = -1;

@@ -163,8 +163,11 @@ __global__ void hist_unit_kernel(HistArgs a, int64_t nbins) {
 
 template <typename R>
 __global__ void hist_bins_kernel(HistArgs a) {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n; p += (int64_t)gridDim.x * blockDim.x)
-    a.bin_of[p] = bin_index<R>(a, p);
+  const uint32_t none = (uint32_t)((int64_t)a.nb[0] * a.nb[1] * a.nb[2]);
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.n; p += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = bin_index<R>(a, p);
+    a.bin_of[p] = b < 0 ? none : (uint32_t)b;
+  }
 }
 
 static int hist_blocks(int64_t n, int threads) {

@@ -90,7 +90,7 @@ struct HistArgs {
   int32_t nb[3];
   int active_dim[3];
   unsigned int *counts32;  // unit-mass path (zeroed)
-  int64_t *bin_of;         // ordered path: per particle bin (or -1), may be null
+  uint32_t *bin_of;        // ordered path: per particle bin, or the number of bins for none
   unsigned long long *nbinned;
 };
 
@@ -123,9 +123,9 @@ cudaError_t sink_record_arrays(void *scratch, int64_t n, int32_t **obs, uint64_t
 cudaError_t launch_resident(const ObsArgs &a, unsigned long long *count, double *msum, cudaStream_t s);
 
 // Ordered (order-preserving) weighted sums: sort.cu
-cudaError_t ordered_bin_sums(const int64_t *bin_of, const double *mass, const int32_t *status, int64_t n,
-                             int64_t nbins, double *counts, double *total_mass, double *sum_w2,
-                             void **scratch, size_t *scratch_bytes, cudaStream_t s);
+// (bins the particles of a.n, a.status; a.bin_of is scratch)
+cudaError_t ordered_bin_sums(HistArgs a, const double *mass, int64_t nbins, double *counts, double *total_mass,
+                             double *sum_w2, void **scratch, size_t *scratch_bytes, cudaStream_t s);
 // processing order: by cell, or -- given the random counters at the start of
 // the previous advance -- heaviest first in buckets of kPassBucket passes
 // of that advance, by cell within a bucket
