@@ -33,6 +33,7 @@ namespace mprw {
 namespace {
 
 constexpr int kAdjThreads = 128;
+constexpr int kWalkThreads = 32;  // one warp per block, as the reverse sweep
 
 __host__ __device__ __forceinline__ int64_t node_id(const AdjGrid &G, int a, int b, int c) {
   return (int64_t)a + (int64_t)(G.n[0] + 1) * ((int64_t)b + (int64_t)(G.n[1] + 1) * c);
@@ -164,16 +165,28 @@ __global__ void adj_node_div_kernel(AdjGrid G, const double *phi, const double *
 }
 
 // ---- one step ----------------------------------------------------------------
+// Both sweeps are bound by the FP64 pipe (a warp instruction holds it for 16
+// clocks; 89 % active at 247 FP64 instructions per walk step and 760 per
+// reverse step), so they take quotients and roots from the integer pipe (the
+// same bits), compares from bit patterns, and multiply by the reciprocal of a
+// cell size that is a power of two (exact): 145 and 430 instructions, 100,000
+// particles 1.03 -> 0.59 ms and 3.18 -> 1.83 ms per 20 steps (84 % active).
+__device__ __forceinline__ double sqrt_i(double x) { return fb::sqrt_plain(x) ? fb::sqrt_core(x) : sqrt(x); }
+__device__ __forceinline__ double div_i(double a, double b) {
+  return fb::div_plain(a, b) ? fb::div_core(a, b, 0) : a / b;
+}
+
 // The cell of a position and its local coordinates (the position is inside
 // the domain after the fold; the last cell takes the upper face).
 __device__ __forceinline__ void locate(const AdjGrid &G, const double x[3], int c[3], double f[3]) {
   for (int d = 0; d < 3; ++d) {
-    const double t = (x[d] - G.lo[d]) / G.d[d];
-    int i = (int)floor(t);
+    const double e = x[d] - G.lo[d];
+    const double t = G.inv_d[d] != 0.0 ? e * G.inv_d[d] : div_i(e, G.d[d]);
+    int i = __double2int_rd(t);
     if (i < 0) i = 0;
     if (i > G.n[d] - 1) i = G.n[d] - 1;
     double fr = t - (double)i;
-    fr = fr < 0.0 ? 0.0 : (fr > 1.0 ? 1.0 : fr);
+    fr = fb::below0(fr) ? 0.0 : (fb::above1(fr) ? 1.0 : fr);
     c[d] = i;
     f[d] = fr;
   }
@@ -182,8 +195,13 @@ __device__ __forceinline__ void locate(const AdjGrid &G, const double x[3], int 
 // reflection at both walls of [lo, lo + L] (a triangle wave: continuous,
 // slope +1 or -1, returned in sgn)
 __device__ __forceinline__ double fold(double y, double lo, double L, double &sgn) {
-  const double P = 2.0 * L;
   double t = y - lo;
+  // inside the walls (L > 0: the bits of [+0, L] are ordered as its values)
+  if (fb::bits(t) <= fb::bits(L)) {
+    sgn = 1.0;
+    return lo + t;
+  }
+  const double P = 2.0 * L;
   t -= floor(t / P) * P;
   if (t > L) {
     sgn = -1.0;
@@ -203,6 +221,23 @@ __device__ __forceinline__ int64_t corner_node(const AdjGrid &G, int64_t base, i
   return base + (o & 1) + (int64_t)(G.n[0] + 1) * (((o >> 1) & 1) + (int64_t)(G.n[1] + 1) * ((o >> 2) & 1));
 }
 
+// a node record: 16-byte loads (records are ADJ_NV = 10 doubles apart)
+struct Node {
+  double v[ADJ_NV];
+};
+__device__ __forceinline__ Node load_node(const double *nodes, int64_t i) {
+  static_assert(ADJ_NV % 2 == 0, "16-byte loads");
+  Node r;
+  const double2 *p = reinterpret_cast<const double2 *>(nodes + ADJ_NV * i);
+#pragma unroll
+  for (int k = 0; k < ADJ_NV / 2; ++k) {
+    const double2 q = __ldg(p + k);
+    r.v[2 * k] = q.x;
+    r.v[2 * k + 1] = q.y;
+  }
+  return r;
+}
+
 __device__ __forceinline__ void interp(const AdjGrid &G, const double *nodes, const int c[3], const double f[3],
                                        Interp &I) {
   I.base = node_id(G, c[0], c[1], c[2]);
@@ -213,25 +248,15 @@ __device__ __forceinline__ void interp(const AdjGrid &G, const double *nodes, co
     const double w = ((o & 1) ? f[0] : 1.0 - f[0]) * (((o >> 1) & 1) ? f[1] : 1.0 - f[1]) *
                      (((o >> 2) & 1) ? f[2] : 1.0 - f[2]);
     I.w[o] = w;
-    const double *nd = nodes + ADJ_NV * corner_node(G, I.base, o);
+    const Node nd = load_node(nodes, corner_node(G, I.base, o));
     for (int d = 0; d < 3; ++d) {
-      I.u[d] += w * nd[d];
-      I.g[d] += w * nd[3 + d];
+      I.u[d] += w * nd.v[d];
+      I.g[d] += w * nd.v[3 + d];
     }
-    I.aL += w * nd[6];
-    I.aT += w * nd[7];
-    I.dm += w * nd[8];
+    I.aL += w * nd.v[6];
+    I.aT += w * nd.v[7];
+    I.dm += w * nd.v[8];
   }
-}
-
-// gradient of corner o's weight
-__device__ __forceinline__ void weight_grad(const AdjGrid &G, const double f[3], int o, double gw[3]) {
-  const double fx = (o & 1) ? f[0] : 1.0 - f[0], fy = ((o >> 1) & 1) ? f[1] : 1.0 - f[1],
-               fz = ((o >> 2) & 1) ? f[2] : 1.0 - f[2];
-  const double sx = (o & 1) ? 1.0 : -1.0, sy = ((o >> 1) & 1) ? 1.0 : -1.0, sz = ((o >> 2) & 1) ? 1.0 : -1.0;
-  gw[0] = sx / G.d[0] * fy * fz;
-  gw[1] = sy / G.d[1] * fx * fz;
-  gw[2] = sz / G.d[2] * fx * fy;
 }
 
 struct Disp {
@@ -241,12 +266,12 @@ struct Disp {
 // B xi = a xi + kappa (u . xi) u
 __device__ __forceinline__ void displacement(const AdjGrid &G, const Interp &I, const double xi[3], Disp &D) {
   D.s2 = I.u[0] * I.u[0] + I.u[1] * I.u[1] + I.u[2] * I.u[2];
-  D.r = sqrt(D.s2 + G.eps2);
+  D.r = sqrt_i(D.s2 + G.eps2);
   const double lt = I.aT * D.r + I.dm;
-  const double ll = lt + (I.aL - I.aT) * D.s2 / D.r;
-  D.a = sqrt(2.0 * lt);
-  D.b = sqrt(2.0 * ll);
-  D.kappa = 2.0 * (I.aL - I.aT) / (D.r * (D.a + D.b));
+  const double ll = lt + div_i((I.aL - I.aT) * D.s2, D.r);
+  D.a = sqrt_i(2.0 * lt);
+  D.b = sqrt_i(2.0 * ll);
+  D.kappa = div_i(2.0 * (I.aL - I.aT), D.r * (D.a + D.b));
   D.P = I.u[0] * xi[0] + I.u[1] * xi[1] + I.u[2] * xi[2];
   for (int d = 0; d < 3; ++d) D.bxi[d] = D.a * xi[d] + D.kappa * D.P * I.u[d];
 }
@@ -272,7 +297,7 @@ __device__ __forceinline__ void step_forward(const AdjGrid &G, const double *nod
   }
 }
 
-__global__ void __launch_bounds__(kAdjThreads) adj_walk_kernel(AdjGrid G, const double *nodes, int64_t np,
+__global__ void __launch_bounds__(kWalkThreads) adj_walk_kernel(AdjGrid G, const double *nodes, int64_t np,
                                                                const uint64_t *id, uint64_t seed, int64_t step0,
                                                                int nst, double dt, const double *xin, double *xout,
                                                                double *seg) {
@@ -392,13 +417,11 @@ __global__ void adj_deposit_adj_kernel(DepGrid Q, int64_t np, const double *x, c
 // Adjoint of x' = fold(x + (u + G) dt + B xi sqrt(dt)) at one step, given
 // lam' = dL/dx'.  Returns lam = dL/dx in lam and adds w_o * (du, dG, daL,
 // daT) of every corner o to acc (8 values per corner; acc belongs to the
-// particle's current cell: the caller flushes it on a cell change).
+// particle's current cell: the caller flushes it on a cell change).  acc is
+// the lane's column in shared memory, entry k at acc[k * stride].
 __device__ __forceinline__ void step_reverse(const AdjGrid &G, const double *nodes, const double x[3],
-                                             const double xi[3], double dt, double sdt, double lam[3],
-                                             double acc[64]) {
-  int c[3];
-  double f[3];
-  locate(G, x, c, f);
+                                             const int c[3], const double f[3], const double xi[3], double dt,
+                                             double sdt, double lam[3], double *acc, int stride) {
   Interp I;
   interp(G, nodes, c, f, I);
   Disp D;
@@ -408,73 +431,98 @@ __device__ __forceinline__ void step_reverse(const AdjGrid &G, const double *nod
     const double y = x[d] + (I.u[d] + I.g[d]) * dt + D.bxi[d] * sdt;
     double sg;
     (void)fold(y, G.lo[d], G.n[d] * G.d[d], sg);
-    lt[d] = sg * lam[d];
+    lt[d] = fb::below0(sg) ? -lam[d] : lam[d];
   }
   // B xi = a xi + kappa P u as a function of u, aL, aT, dm: the transposed
   // derivatives applied to lt.  With r = sqrt(|u|^2 + eps^2): da = (aT / a)
   // dr, dr = (u . du) / r, db = d(ll) / b, dkappa = -kappa (dr / r + (da + db)
-  // / (a + b)).
+  // / (a + b)).  Four reciprocals serve every quotient.
   const double ul = I.u[0] * lt[0] + I.u[1] * lt[1] + I.u[2] * lt[2];
   const double xl = xi[0] * lt[0] + xi[1] * lt[1] + xi[2] * lt[2];
-  const double r = D.r, a = D.a, b = D.b, k = D.kappa, P = D.P, s2 = D.s2, ab = a + b;
-  const double dA = I.aL - I.aT;
-  const double ca = (I.aT / a) / r;                                          // da = ca (u . du)
-  const double cb = (I.aT / r + dA * (2.0 / r - s2 / (r * r * r))) / b;      // db = cb (u . du)
-  const double ck = -k * (1.0 / (r * r) + (ca + cb) / ab);                   // dkappa = ck (u . du)
-  double jv[3];
-  for (int d = 0; d < 3; ++d) jv[d] = ca * xl * I.u[d] + ck * P * ul * I.u[d] + k * ul * xi[d] + k * P * lt[d];
-  const double dk_daL = 2.0 / (r * ab) - k * (s2 / (r * b)) / ab;
-  const double da_daT = r / a, db_daT = (r - s2 / r) / b;
-  const double dk_daT = -2.0 / (r * ab) - k * (da_daT + db_daT) / ab;
-  const double dk_ddm = -k * (1.0 / a + 1.0 / b) / ab;
-  const double cL = dk_daL * P * ul;
-  const double cT = da_daT * xl + dk_daT * P * ul;
-  const double cD = xl / a + dk_ddm * P * ul;
-  double ln[3] = {lt[0], lt[1], lt[2]};
+  const double k = D.kappa, P = D.P, s2 = D.s2, dA = I.aL - I.aT;
+  const double ir = div_i(1.0, D.r), ia = div_i(1.0, D.a), ib = div_i(1.0, D.b), iab = div_i(1.0, D.a + D.b);
+  const double ir2 = ir * ir, s2r = s2 * ir;
+  const double ca = I.aT * ia * ir;                                          // da = ca (u . du)
+  const double cb = (I.aT * ir + dA * (2.0 * ir - s2r * ir2)) * ib;          // db = cb (u . du)
+  const double ck = -k * (ir2 + (ca + cb) * iab);                            // dkappa = ck (u . du)
+  const double Pul = P * ul, ju = ca * xl + ck * Pul, jx = k * ul, jl = k * P;
+  const double da_daT = D.r * ia, db_daT = (D.r - s2r) * ib;
+  const double cL = ir * iab * (2.0 - k * s2 * ib) * Pul;
+  const double cT = da_daT * xl - iab * (2.0 * ir + k * (da_daT + db_daT)) * Pul;
+  const double cD = xl * ia - k * (ia + ib) * iab * Pul;
+  // dL/d(field) of the interpolated u, G, aL, aT, Dm
+  double q[9];
+  for (int d = 0; d < 3; ++d) {
+    q[3 + d] = dt * lt[d];
+    q[d] = q[3 + d] + sdt * (ju * I.u[d] + jx * xi[d] + jl * lt[d]);
+  }
+  q[6] = sdt * cL;
+  q[7] = sdt * cT;
+  q[8] = sdt * cD;
+  double s[8];  // per corner: q . node values
 #pragma unroll
   for (int o = 0; o < 8; ++o) {
     const double w = I.w[o];
-    double *A = acc + 8 * o;
-    for (int d = 0; d < 3; ++d) {
-      A[d] += w * (dt * lt[d] + sdt * jv[d]);
-      A[3 + d] += w * (dt * lt[d]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      double *A = acc + (8 * o + j) * stride;
+      *A += w * q[j];
     }
-    A[6] += w * sdt * cL;
-    A[7] += w * sdt * cT;
-    const double *nd = nodes + ADJ_NV * corner_node(G, I.base, o);
-    const double s = dt * ((nd[0] + nd[3]) * lt[0] + (nd[1] + nd[4]) * lt[1] + (nd[2] + nd[5]) * lt[2]) +
-                     sdt * (nd[0] * jv[0] + nd[1] * jv[1] + nd[2] * jv[2] + nd[6] * cL + nd[7] * cT + nd[8] * cD);
-    double gw[3];
-    weight_grad(G, f, o, gw);
-    for (int d = 0; d < 3; ++d) ln[d] += s * gw[d];
+    const Node nd = load_node(nodes, corner_node(G, I.base, o));
+    double t = q[0] * nd.v[0];
+#pragma unroll
+    for (int j = 1; j < 9; ++j) t += q[j] * nd.v[j];
+    s[o] = t;
   }
-  for (int d = 0; d < 3; ++d) lam[d] = ln[d];
+  // the weights' gradients: along an axis, the corner differences times the
+  // other two axes' weights
+  const double gx = 1.0 - f[0], gy = 1.0 - f[1], gz = 1.0 - f[2];
+  const double dx = gz * (gy * (s[1] - s[0]) + f[1] * (s[3] - s[2])) +
+                    f[2] * (gy * (s[5] - s[4]) + f[1] * (s[7] - s[6]));
+  const double dy = gz * (gx * (s[2] - s[0]) + f[0] * (s[3] - s[1])) +
+                    f[2] * (gx * (s[6] - s[4]) + f[0] * (s[7] - s[5]));
+  const double dz = gy * (gx * (s[4] - s[0]) + f[0] * (s[5] - s[1])) +
+                    f[1] * (gx * (s[6] - s[2]) + f[0] * (s[7] - s[3]));
+  lam[0] = lt[0] + dx * G.rec_d[0];
+  lam[1] = lt[1] + dy * G.rec_d[1];
+  lam[2] = lt[2] + dz * G.rec_d[2];
 }
 
-__device__ __forceinline__ void flush_acc(const AdjGrid &G, int64_t base, double acc[64], double *nadj) {
+__device__ __forceinline__ void flush_acc(const AdjGrid &G, int64_t base, double *acc, int stride, double *nadj) {
   if (base < 0) return;
-#pragma unroll
+#pragma unroll 1
   for (int o = 0; o < 8; ++o) {
     double *dst = nadj + 8 * corner_node(G, base, o);
+#pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const double v = acc[8 * o + k];
-      if (v != 0.0) atomicAdd(dst + k, v);
-      acc[8 * o + k] = 0.0;
+      double *A = acc + (8 * o + k) * stride;
+      const double v = *A;
+      if (!fb::is0(v)) atomicAdd(dst + k, v);
+      *A = 0.0;
     }
   }
 }
 
-__global__ void __launch_bounds__(kAdjThreads) adj_reverse_kernel(AdjGrid G, const double *nodes, int64_t np,
-                                                                  const uint64_t *id, uint64_t seed, int64_t step0,
-                                                                  int nst, double dt, const double *seg,
-                                                                  double *lam_io, double *nadj) {
-  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// One warp per block (kAdjWarp): a block's whole work is one warp's, so the
+// SMs even out at the end (782 blocks of four warps left a sixth of the time
+// to the last wave).  The 64 accumulators of a lane's cell are its column of
+// the block's shared memory (16 KB): in local memory they and their spills
+// took 381 load/store instructions per step.
+constexpr int kAdjWarp = 32;
+
+__global__ void __launch_bounds__(kAdjWarp) adj_reverse_kernel(AdjGrid G, const double *nodes, int64_t np,
+                                                               const uint64_t *id, uint64_t seed, int64_t step0,
+                                                               int nst, double dt, const double *seg,
+                                                               double *lam_io, double *nadj) {
+  __shared__ double acc_all[64 * kAdjWarp];
+  double *acc = acc_all + threadIdx.x;
+  const int64_t p = blockIdx.x * (int64_t)kAdjWarp + threadIdx.x;
+  const unsigned warp = __ballot_sync(0xffffffffu, p < np);
   if (p >= np) return;
   double lam[3] = {lam_io[p], lam_io[np + p], lam_io[2 * np + p]};
   const double sdt = sqrt(dt);
   const uint64_t pid = id[p];
-  double acc[64];
-  for (int k = 0; k < 64; ++k) acc[k] = 0.0;
+  for (int k = 0; k < 64; ++k) acc[k * kAdjWarp] = 0.0;
   int64_t base = -1;
   for (int k = nst - 1; k >= 0; --k) {
     const double x[3] = {seg[((int64_t)k * 3 + 0) * np + p], seg[((int64_t)k * 3 + 1) * np + p],
@@ -484,14 +532,15 @@ __global__ void __launch_bounds__(kAdjThreads) adj_reverse_kernel(AdjGrid G, con
     locate(G, x, c, f);
     const int64_t b = node_id(G, c[0], c[1], c[2]);
     if (b != base) {
-      flush_acc(G, base, acc, nadj);
+      flush_acc(G, base, acc, kAdjWarp, nadj);
       base = b;
     }
+    __syncwarp(warp);  // the lanes that flushed rejoin (left apart, 3 lanes ran together)
     double xi[3];
     normals(seed, pid, step0 + k, xi);
-    step_reverse(G, nodes, x, xi, dt, sdt, lam, acc);
+    step_reverse(G, nodes, x, c, f, xi, dt, sdt, lam, acc, kAdjWarp);
   }
-  flush_acc(G, base, acc, nadj);
+  flush_acc(G, base, acc, kAdjWarp, nadj);
   for (int d = 0; d < 3; ++d) lam_io[d * np + p] = lam[d];
 }
 
@@ -685,6 +734,9 @@ cudaError_t AdjState::setup(const AdjInputs &in, const AdjOptions &opt, const in
   for (int d = 0; d < 3; ++d) {
     G.lo[d] = in.lo[d];
     G.d[d] = in.d[d];
+    int ex = 0;
+    G.rec_d[d] = 1.0 / in.d[d];
+    G.inv_d[d] = std::frexp(in.d[d], &ex) == 0.5 ? G.rec_d[d] : 0.0;
   }
   G.nnode = (int64_t)(G.n[0] + 1) * (G.n[1] + 1) * (G.n[2] + 1);
   G.eps2 = opt.eps * opt.eps;
@@ -752,11 +804,11 @@ cudaError_t AdjState::forward(const double *theta_host, double *density_host, cu
   adj_node_div_kernel<<<nb, kAdjThreads, 0, s>>>(G, d_phi, d_phid, d_nodes);
   launches = 2;
   const int nseg = (o.nsteps + o.checkpoint - 1) / o.checkpoint;
-  const int pb = (int)((np + kAdjThreads - 1) / kAdjThreads);
+  const int pb = (int)((np + kWalkThreads - 1) / kWalkThreads);
   for (int j = 0; j < nseg && np > 0; ++j) {
     const int64_t step0 = (int64_t)j * o.checkpoint;
     const int nst = (int)std::min<int64_t>(o.checkpoint, o.nsteps - step0);
-    adj_walk_kernel<<<pb, kAdjThreads, 0, s>>>(G, d_nodes, np, d_id, o.seed, step0, nst, o.dt,
+    adj_walk_kernel<<<pb, kWalkThreads, 0, s>>>(G, d_nodes, np, d_id, o.seed, step0, nst, o.dt,
                                                 d_ckpt + (size_t)j * 3 * np, d_ckpt + (size_t)(j + 1) * 3 * np,
                                                 nullptr);
     ++launches;
@@ -796,14 +848,14 @@ cudaError_t AdjState::backward(const double *gdens_host, double *grad_host, cuda
     ++launches;
   }
   ACK(cudaMemsetAsync(d_nadj, 0, sizeof(double) * 8 * G.nnode, s));
-  const int pb = (int)((np + kAdjThreads - 1) / kAdjThreads);
+  const int pb = (int)((np + kWalkThreads - 1) / kWalkThreads);
   for (int j = nseg - 1; j >= 0 && np > 0; --j) {
     const int64_t step0 = (int64_t)j * o.checkpoint;
     const int nst = (int)std::min<int64_t>(o.checkpoint, o.nsteps - step0);
     // recompute the segment from its checkpoint, storing the position before every step
-    adj_walk_kernel<<<pb, kAdjThreads, 0, s>>>(G, d_nodes, np, d_id, o.seed, step0, nst, o.dt,
+    adj_walk_kernel<<<pb, kWalkThreads, 0, s>>>(G, d_nodes, np, d_id, o.seed, step0, nst, o.dt,
                                                 d_ckpt + (size_t)j * 3 * np, nullptr, d_seg);
-    adj_reverse_kernel<<<pb, kAdjThreads, 0, s>>>(G, d_nodes, np, d_id, o.seed, step0, nst, o.dt, d_seg, d_lam,
+    adj_reverse_kernel<<<pb, kAdjWarp, 0, s>>>(G, d_nodes, np, d_id, o.seed, step0, nst, o.dt, d_seg, d_lam,
                                                    d_nadj);
     launches += 2;
   }

@@ -45,12 +45,13 @@
 namespace mprw {
 
 constexpr int ADJ_MAXZONES = 64;
-constexpr int ADJ_NV = 9;  // node record: u[3], g[3], alphaL, alphaT, Dm/R
+constexpr int ADJ_NV = 10;  // node record: u[3], g[3], alphaL, alphaT, Dm/R (and padding to 16 bytes)
 
 struct AdjGrid {
   int n[3];       // cells along model x, y, z
   double lo[3];   // domain corner (model coordinates)
   double d[3];    // cell size
+  double rec_d[3], inv_d[3];  // 1 / cell size; the same where it is exact (a power of two), else 0
   int64_t nnode;  // (n0+1)(n1+1)(n2+1)
   double eps2;    // velocity floor squared
 };
