@@ -95,6 +95,35 @@ MPRW_FB bool past_end(double maxTime, double t) {
   return maxTime < t;
 }
 
+// |a b| > 1/2, the product rounded: from the exponents, and where those leave
+// it open (significands whose product decides between 1/4 and 1) from the
+// significands' leading 32 bits; the product itself only within 2^-29 of 1/2.
+MPRW_FB unsigned mulhi_u(unsigned a, unsigned b) {
+#if defined(__CUDA_ARCH__)
+  return __umulhi(a, b);
+#else
+  return (unsigned)(((unsigned long long)a * b) >> 32);
+#endif
+}
+MPRW_FB bool prod_above_half(double a, double b) {
+  const unsigned long long ba = bits(a), bb = bits(b);
+  const int ea = (int)((ba >> 52) & 0x7FF), eb = (int)((bb >> 52) & 0x7FF);
+  const int e = ea + eb - 2046;  // |a b| in [2^e, 2^(e+2)) for normal a, b
+  if ((unsigned)(ea - 1) < 2046u && (unsigned)(eb - 1) < 2046u) {
+    if (e >= 0) return true;
+    if (e <= -3) return false;
+    const unsigned ha = 0x80000000u | (unsigned)((ba >> 21) & 0x7FFFFFFFu);
+    const unsigned hb = 0x80000000u | (unsigned)((bb >> 21) & 0x7FFFFFFFu);
+    const unsigned p = mulhi_u(ha, hb);  // significands' product in 2^-30, less than 3 units low
+    const unsigned half = e == -1 ? 0x40000000u : 0x80000000u;
+    if (p > half) return true;
+    if (p < half - 3u) return false;
+  } else if ((ba << 1) == 0ULL && eb < 2047) {
+    return false;
+  }
+  return abs_above_half(a * b);
+}
+
 MPRW_FB int clz64(unsigned long long m) {
 #if defined(__CUDA_ARCH__)
   return __clzll((long long)m);

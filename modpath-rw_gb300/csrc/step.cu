@@ -21,8 +21,7 @@
 
 namespace mprw {
 
-// Shared-memory view of one lane's record: field f at sm[f*stride + lane],
-// conflict-free for a warp reading the same field.
+// Shared-memory view of one lane's record: field f at sm[f].
 enum : int {
   F_V1 = 0, F_DV = 3, F_D = 6, F_INVD = 9, F_DIV = 12, F_VB = 33,
   F_AL = 57, F_AT = 58, F_DM = 59, F_2R = 60, F_V2 = 61, F_ALV = 64, F_ATV = 65, NFIELDS = 66
@@ -31,8 +30,8 @@ enum : int {
 template <typename R>
 struct Lane {
   R *p;
-  int stride;
-  __device__ __forceinline__ R operator()(int f) const { return p[f * stride]; }
+  int stride;  // threads of the block
+  __device__ __forceinline__ R operator()(int f) const { return p[f]; }
 };
 
 // Tests against the constants 0, 1/2 and 1 and the time compares: native in
@@ -65,6 +64,13 @@ template <typename R>
 __device__ __forceinline__ bool abs_above_half(R v) { return fabs(v) > R(0.5); }
 template <>
 __device__ __forceinline__ bool abs_above_half<double>(double v) { return fb::abs_above_half(v); }
+// |a b| > 1/2: in the FP64 kernel without the product (the jump limiter's test
+// of every pass; 54.7 -> 52.3 ms on the same workload, with the exit steps
+// formed on two axes 51.8)
+template <typename R>
+__device__ __forceinline__ bool over_half(R a, R b) { return fabs(a * b) > R(0.5); }
+template <>
+__device__ __forceinline__ bool over_half<double>(double a, double b) { return fb::prod_above_half(a, b); }
 template <typename R>
 __device__ __forceinline__ bool out01(R v) { return v > R(1) || v < R(0); }
 template <>
@@ -99,64 +105,78 @@ using fb::eq_any;
 using fb::lt_any;
 using fb::past_end;
 
-// The staged fields are the record's first NFIELDS values and records are
-// 16-byte aligned, so they are read with 16-byte loads (FP32: 16 float4 and
-// one float2; FP64: 33 double2) and scattered to the lane's SoA slots.
-static_assert(NFIELDS == 66, "stage_record reads 66 leading fields");
+// A lane's record in shared memory: the cell record's first NFIELDS values as
+// they are (and, in FP32, two more words), kRecBytes apart -- an odd number of
+// 16-byte units, so that 16-byte reads of one field pair by all lanes meet no
+// bank twice.
+static_assert(NFIELDS == 66, "the record's leading fields");
 template <typename R>
-__device__ __forceinline__ void stage_record(const CellRec<R> *__restrict__ recs, int32_t c, R *sm, int stride);
+constexpr int kRecUnits = sizeof(R) == 8 ? 33 : 17;
+template <typename R>
+constexpr int kRecStride = kRecUnits<R> * 16 / (int)sizeof(R);
 
-template <>
-__device__ __forceinline__ void stage_record<float>(const CellRec<float> *__restrict__ recs, int32_t c, float *sm,
-                                                    int stride) {
-  const float4 *src = reinterpret_cast<const float4 *>(recs + c);
-#pragma unroll 4
-  for (int q = 0; q < 16; ++q) {
-    const float4 v = __ldg(src + q);
-    sm[(4 * q + 0) * stride] = v.x;
-    sm[(4 * q + 1) * stride] = v.y;
-    sm[(4 * q + 2) * stride] = v.z;
-    sm[(4 * q + 3) * stride] = v.w;
+// Asynchronous copies, all in flight at once and without a register each;
+// stage_wait before the first read.  Every warp waits here for its entering
+// lanes in nine iterations of ten: loads and stores of one field column per
+// lane (17 or 33 loads, 66 stores, in batches), after the entry checks, held
+// MIXED at 12.5 ms and FP64 at 50.9 ms over three 10-day intervals of 1,000,000
+// particles in the lognormal slab; these, issued before the checks, 10.7 and
+// 50.5.
+template <typename R>
+__device__ __forceinline__ void stage_record(const CellRec<R> *__restrict__ recs, int32_t c, R *sm) {
+  const char *src = reinterpret_cast<const char *>(recs + c);
+  const unsigned dst = (unsigned)__cvta_generic_to_shared(sm);
+#pragma unroll
+  for (int q = 0; q < kRecUnits<R>; ++q)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * q), "l"(src + 16 * q) : "memory");
+}
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// N consecutive fields from a 16-byte boundary-aligned window (fields before
+// base in the first unit and after the last are dropped)
+template <typename R, int BASE, int N>
+__device__ __forceinline__ void fields(const Lane<R> &F, R (&v)[N]) {
+  constexpr int K = 16 / (int)sizeof(R), U0 = BASE / K, U1 = (BASE + N + K - 1) / K;
+#pragma unroll
+  for (int u = U0; u < U1; ++u) {
+    if constexpr (sizeof(R) == 8) {
+      const double2 q = reinterpret_cast<const double2 *>(F.p)[u];
+      const double t[2] = {q.x, q.y};
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (u * K + k >= BASE && u * K + k < BASE + N) v[u * K + k - BASE] = t[k];
+    } else {
+      const float4 q = reinterpret_cast<const float4 *>(F.p)[u];
+      const float t[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (u * K + k >= BASE && u * K + k < BASE + N) v[u * K + k - BASE] = t[k];
+    }
   }
-  const float2 t = __ldg(reinterpret_cast<const float2 *>(src + 16));
-  sm[64 * stride] = t.x;
-  sm[65 * stride] = t.y;
 }
 
-template <>
-__device__ __forceinline__ void stage_record<double>(const CellRec<double> *__restrict__ recs, int32_t c,
-                                                     double *sm, int stride) {
-  const double2 *src = reinterpret_cast<const double2 *>(recs + c);
-#pragma unroll 4
-  for (int q = 0; q < 33; ++q) {
-    const double2 v = __ldg(src + q);
-    sm[(2 * q + 0) * stride] = v.x;
-    sm[(2 * q + 1) * stride] = v.y;
-  }
-}
-
 template <typename R>
-__device__ __forceinline__ R tril(const Lane<R> &F, int base, R x, R y, R z, R xy, R xz, R yz, R xyz) {
-  R a = F(base + 0);
-  a = fma(F(base + 1), x, a);
-  a = fma(F(base + 2), y, a);
-  a = fma(F(base + 3), z, a);
-  a = fma(F(base + 4), xy, a);
-  a = fma(F(base + 5), xz, a);
-  a = fma(F(base + 6), yz, a);
-  a = fma(F(base + 7), xyz, a);
+__device__ __forceinline__ R tril(const R *c, R x, R y, R z, R xy, R xz, R yz, R xyz) {
+  R a = c[0];
+  a = fma(c[1], x, a);
+  a = fma(c[2], y, a);
+  a = fma(c[3], z, a);
+  a = fma(c[4], xy, a);
+  a = fma(c[5], xz, a);
+  a = fma(c[6], yz, a);
+  a = fma(c[7], xyz, a);
   return a;
 }
 
 template <typename R>
-__device__ __forceinline__ R divc(const Lane<R> &F, int base, R x, R y, R z, R xy, R xz, R yz) {
-  R a = F(base + 0);
-  a = fma(F(base + 1), x, a);
-  a = fma(F(base + 2), y, a);
-  a = fma(F(base + 3), z, a);
-  a = fma(F(base + 4), xy, a);
-  a = fma(F(base + 5), xz, a);
-  a = fma(F(base + 6), yz, a);
+__device__ __forceinline__ R divc(const R *c, R x, R y, R z, R xy, R xz, R yz) {
+  R a = c[0];
+  a = fma(c[1], x, a);
+  a = fma(c[2], y, a);
+  a = fma(c[3], z, a);
+  a = fma(c[4], xy, a);
+  a = fma(c[5], xz, a);
+  a = fma(c[6], yz, a);
   return a;
 }
 
@@ -206,9 +226,11 @@ __device__ __forceinline__ void random_displacement(const Lane<R> &F, int ndim, 
     aT = F(F_ATV) + cosinesq * (aTH - F(F_ATV));
   }
   if (ndim == 3) {
-    R vx = tril(F, F_VB + 0, x, y, z, xy, xz, yz, xyz);
-    R vy = tril(F, F_VB + 8, x, y, z, xy, xz, yz, xyz);
-    R vz = tril(F, F_VB + 16, x, y, z, xy, xz, yz, xyz);
+    R cv[24];
+    fields<R, F_VB, 24>(F, cv);
+    R vx = tril(cv, x, y, z, xy, xz, yz, xyz);
+    R vy = tril(cv + 8, x, y, z, xy, xz, yz, xyz);
+    R vz = tril(cv + 16, x, y, z, xy, xz, yz, xyz);
     R nxy2 = fma(vx, vx, vy * vy);
     R n2 = fma(vz, vz, nxy2);
     R B11 = zero, B12 = zero, B13 = zero, B21 = zero, B22 = zero, B23 = zero, B31 = zero, B32 = zero;
@@ -241,8 +263,8 @@ __device__ __forceinline__ void random_displacement(const Lane<R> &F, int ndim, 
     by = fma(B23, rz, fma(B22, ry, B21 * rx));
     bz = fma(B32, ry, B31 * rx);
   } else if (ndim == 2) {
-    R v1 = tril(F, F_VB + 8 * d1, x, y, z, xy, xz, yz, xyz);
-    R v2 = tril(F, F_VB + 8 * d2, x, y, z, xy, xz, yz, xyz);
+    R v1 = tril(F.p + F_VB + 8 * d1, x, y, z, xy, xz, yz, xyz);
+    R v2 = tril(F.p + F_VB + 8 * d2, x, y, z, xy, xz, yz, xyz);
     R n2 = fma(v1, v1, v2 * v2);
     R B11 = zero, B12 = zero, B21 = zero, B22 = zero;
     if (n2 > zero) {
@@ -262,7 +284,7 @@ __device__ __forceinline__ void random_displacement(const Lane<R> &F, int ndim, 
     if (d1 == 0) bx = o1; else if (d1 == 1) by = o1; else bz = o1;
     if (d2 == 0) bx = o2; else if (d2 == 1) by = o2; else bz = o2;
   } else {
-    R v1 = tril(F, F_VB + 8 * d1, x, y, z, xy, xz, yz, xyz);
+    R v1 = tril(F.p + F_VB + 8 * d1, x, y, z, xy, xz, yz, xyz);
     R nrm = fabs(v1);
     R B11 = zero;
     if (nrm > zero) B11 = sqrt_r(tr * fma(aL, nrm, dm));
@@ -757,7 +779,7 @@ __device__ __forceinline__ void warp_exit_solves(unsigned grp, unsigned need, co
   // this lane's own tasks, one per leaving axis
   const int t0 = __popc(m0 & below), t1 = c0 + __popc(m1 & below), t2 = c0 + c1 + __popc(m2 & below);
   double *slot = slots + (threadIdx.x & ~31);  // the warp's slots
-  const R *rec = F.p - lane;                   // the warp's records
+  const R *rec = F.p - lane * kRecStride<R>;   // the warp's records
   rbits = 0u;
   tx = ty = tz = 0.0;
   fx = fy = fz = 0;
@@ -782,7 +804,7 @@ __device__ __forceinline__ void warp_exit_solves(unsigned grp, unsigned need, co
       const int a = (meta >> 5) & 3;
       int efa = 0, ef_unused = 0;
       double dta = 0.0, dt_unused = 0.0;
-      const double d = (double)rec[(F_D + a) * stride + (meta & 31)];
+      const double d = (double)rec[(meta & 31) * kRecStride<R> + F_D + a];
       bool r;
       if constexpr (EXP)
         r = newton_axis((meta & 128) != 0, slot[rank], d, slot[stride + rank], slot[6 * stride + rank],
@@ -832,16 +854,20 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t ma
     sdt = sqrt_r(rdt);
   }
   R x = V.x, y = V.y, z = V.z;
-  R dX = F(F_D + 0), dY = F(F_D + 1), dZ = F(F_D + 2);
-  R iX = F(F_INVD + 0), iY = F(F_INVD + 1), iZ = F(F_INVD + 2);
+  R head[12];  // V1, DV, D, 1/D
+  fields<R, 0, 12>(F, head);
+  R dX = head[F_D + 0], dY = head[F_D + 1], dZ = head[F_D + 2];
+  R iX = head[F_INVD + 0], iY = head[F_INVD + 1], iZ = head[F_INVD + 2];
   // pr_RWPTDisplacementsLinear (:673-706)
-  R vx = fma(x, F(F_DV + 0), F(F_V1 + 0));
-  R vy = fma(y, F(F_DV + 1), F(F_V1 + 1));
-  R vz = fma(z, F(F_DV + 2), F(F_V1 + 2));
+  R vx = fma(x, head[F_DV + 0], head[F_V1 + 0]);
+  R vy = fma(y, head[F_DV + 1], head[F_V1 + 1]);
+  R vz = fma(z, head[F_DV + 2], head[F_V1 + 2]);
   R xy = x * y, xz = x * z, yz = y * z;
-  R ddx = divc(F, F_DIV + 0, x, y, z, xy, xz, yz);
-  R ddy = divc(F, F_DIV + 7, x, y, z, xy, xz, yz);
-  R ddz = divc(F, F_DIV + 14, x, y, z, xy, xz, yz);
+  R cd[21];
+  fields<R, F_DIV, 21>(F, cd);
+  R ddx = divc(cd, x, y, z, xy, xz, yz);
+  R ddy = divc(cd + 7, x, y, z, xy, xz, yz);
+  R ddz = divc(cd + 14, x, y, z, xy, xz, yz);
   R bx, by, bz;
   random_displacement<R, AXI>(F, ndim, d1, d2, x, y, z, vx, vy, vz, seed, id, ctr, bx, by, bz);
   // advection displacement: EULERIAN v dt, EXPONENTIAL (FP64) v (e^{dv dt}-1)/dv
@@ -899,7 +925,7 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t ma
       V.reachedMax = false;
     }
   } else
-  while (sizeof(R) == 8 ? abs_above_half(dxrw * iX) | abs_above_half(dyrw * iY) | abs_above_half(dzrw * iZ)
+  while (sizeof(R) == 8 ? over_half(dxrw, iX) | over_half(dyrw, iY) | over_half(dzrw, iZ)
                         : (fabs(dxrw * iX) > half) || (fabs(dyrw * iY) > half) || (fabs(dzrw * iZ) > half)) {
     V.t = V.t - dt;
     dt = dtRed * dt;
@@ -1068,21 +1094,31 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t ma
     }
     if constexpr (sizeof(R) == 8 || EXP) rdt = (R)dt;  // MIXED EULERIAN: rdt set above
     sdt = sqrt_r(rdt);
-    advect();
+    if constexpr (sizeof(R) == 4) advect();
     V.reachedMax = false;
     int ef = V.exitFace;
     if (ef >= 1 && ef <= 6 && sizeof(R) == 8) {
-      // FP64: the step of the truncated time on every axis (one shared
-      // block), then the exit axis pinned to its face
-      const R dxc = ax + ddx * rdt + bx * sdt;
-      const R dyc = ay + ddy * rdt + by * sdt;
-      const R dzc = az + ddz * rdt + bz * sdt;
-      const R nxc = x + dxc * iX, nyc = y + dyc * iY, nzc = z + dzc * iZ;
+      // FP64: the exit axis pinned to its face, the step of the truncated
+      // time on the two others (p and q, one shared block)
       const int fa = (ef - 1) >> 1;
+      const bool p0 = fa != 0, q2 = fa != 2;  // p: x, or y when x is pinned; q: z, or y
       const R pin = (ef & 1) ? zero : one;
-      if (fa != 0) { dxrw = dxc; nx = nxc; } else { nx = pin; }
-      if (fa != 1) { dyrw = dyc; ny = nyc; } else { ny = pin; }
-      if (fa != 2) { dzrw = dzc; nz = nzc; } else { nz = pin; }
+      const double dvp = p0 ? dvx : dvy, dvq = q2 ? dvz : dvy;
+      const R vp = p0 ? vx : vy, vq = q2 ? vz : vy;
+      R ap, aq;
+      if constexpr (EXP) {
+        ap = (R)adv_exponential((double)vp, dvp, dt, exp(dvp * dt) - 1.0);
+        aq = (R)adv_exponential((double)vq, dvq, dt, exp(dvq * dt) - 1.0);
+      } else {
+        ap = vp * rdt;
+        aq = vq * rdt;
+      }
+      const R dp = ap + (p0 ? ddx : ddy) * rdt + (p0 ? bx : by) * sdt;
+      const R dq = aq + (q2 ? ddz : ddy) * rdt + (q2 ? bz : by) * sdt;
+      const R np = (p0 ? x : y) + dp * (p0 ? iX : iY), nq = (q2 ? z : y) + dq * (q2 ? iZ : iY);
+      if (fa == 0) { nx = pin; dyrw = dp; ny = np; dzrw = dq; nz = nq; }
+      else if (fa == 1) { dxrw = dp; nx = np; ny = pin; dzrw = dq; nz = nq; }
+      else { dxrw = dp; nx = np; dyrw = dq; ny = nq; nz = pin; }
     } else if (ef == 1 || ef == 2) {
       nx = (ef == 1) ? zero : one;
       dyrw = ay + ddy * rdt + by * sdt;
@@ -1199,11 +1235,11 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t ma
 template <typename R, bool EXP, bool AXI>
 __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) == 4 && !EXP) ? 3 : 1) rwpt_advance_kernel(AdvanceArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  R *sm = reinterpret_cast<R *>(smraw) + threadIdx.x;
+  R *sm = reinterpret_cast<R *>(smraw) + threadIdx.x * kRecStride<R>;
   const int stride = blockDim.x;
   Lane<R> F{sm, stride};
   // the exchange slots (FP64 or EXPONENTIAL) follow the records
-  double *slots = reinterpret_cast<double *>(reinterpret_cast<R *>(smraw) + NFIELDS * stride);
+  double *slots = reinterpret_cast<double *>(reinterpret_cast<R *>(smraw) + kRecStride<R> * stride);
   const R zero = R(0), one = R(1);
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -1312,28 +1348,31 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
         fin = ST_UNDEFINED;  // InvalidLocation (TrackCell.f90:410-413)
         use_last = true;
       } else {
+        // the record is on its way while the entry checks are read
         const CellRec<R> *rec = a.recs + c;
+        stage_record(a.recs, c, sm);
         const int32_t es = rec->entry_status;
+        const double dtc = rec->dtcell, sdtc = rec->sqrt_dtcell;
+        massb = rec->massb;
+        stage_wait();
         if (es != 0) {
           fin = es;
           use_last = (es == ST_UNDEFINED);
         } else {
-          stage_record(a.recs, c, sm, stride);
           if constexpr (EXP) {
             double *xf = slots + kExitSlot * stride + threadIdx.x;
             for (int d = 0; d < 3; ++d) {
               const double g = div_r((double)F(F_DV + d), (double)F(F_D + d));
               xf[d * stride] = g;
-              xf[(3 + d) * stride] = exp(g * rec->dtcell) - 1.0;
+              xf[(3 + d) * stride] = exp(g * dtc) - 1.0;
             }
           }
-          massb = rec->massb;
           V.x = ex; V.y = ey; V.z = ez;
           V.ix = ex; V.iy = ey; V.iz = ez;
           V.t = et; V.tinit = et;
-          V.dtcell = rec->dtcell;
-          V.sqrt_dtcell = (R)rec->sqrt_dtcell;
-          V.rdt_cell = (R)rec->dtcell;
+          V.dtcell = dtc;
+          V.sqrt_dtcell = (R)sdtc;
+          V.rdt_cell = (R)dtc;
           V.exitFace = 0;
           V.posRestart = 0;
           V.reachedMax = false;
@@ -1426,7 +1465,7 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
 template <typename R>
 static size_t advance_smem_bytes(int threads, int exp_adv) {
   const int extra = exp_adv ? kExitSlot + kExpFields : (sizeof(R) == 8 ? kExitSlot - 1 : 0);
-  return (NFIELDS * sizeof(R) + extra * sizeof(double)) * threads;
+  return (kRecUnits<R> * 16 + extra * sizeof(double)) * threads;
 }
 
 template <typename R>

@@ -30,6 +30,14 @@ static void check_sqrt(double x) {
   if (bits(r) != bits(w) && g_bad++ < 20) std::printf("MISMATCH sqrt(%a) = %a got %a\n", x, r, w);
 }
 
+// |a b| > 1/2 against the rounded product's compare
+static void check_prod(double a, double b) {
+  ++g_checked;
+  volatile double p = a * b;
+  const bool want = std::fabs(p) > 0.5, got = prod_above_half(a, b);
+  if (got != want && g_bad++ < 20) std::printf("MISMATCH |%a * %a| > 1/2: got %d want %d\n", a, b, got, want);
+}
+
 int main() {
   const unsigned long long sig = 0x000FFFFFFFFFFFFFULL;
   std::mt19937_64 rng(20240);
@@ -65,6 +73,21 @@ int main() {
             check_sqrt(a);
           }
   }
+  // products around 1/2 (every exponent sum from 2^-4 to 2^1), at it exactly
+  // and next to it, and with special values
+  for (int i = 0; i < 3000000; ++i) {
+    const unsigned long long ra = rng(), rb = rng();
+    const int e = (int)(ra >> 60) - 8;
+    double a = from_bits(((unsigned long long)(1023 + e) << 52) | (ra & sig));
+    double b = from_bits(((unsigned long long)(1023 - e - 3 + (int)(rb >> 61) % 5) << 52) | (rb & sig));
+    if (i % 3 == 0) b = 0.5 / a;
+    if (i % 3 == 1 && i % 2) b = std::nextafter(0.5 / a, i % 4 == 1 ? 2.0 : 0.0);
+    check_prod(i % 5 ? a : -a, b);
+  }
+  const double special[] = {0.0, -0.0, from_bits(1), 1e-310, 0.5, -0.5, 1.0, -1.0, std::nextafter(1.0, 2.0),
+                            std::nextafter(0.5, 0.0), 2.0, 1e300, 1e-300, INFINITY, -INFINITY, (double)NAN};
+  for (double a : special)
+    for (double b : special) check_prod(a, b);
   // refused operands: zeros, subnormals, infinities, NaN, quotients (or their
   // halves) outside the normal range, negative radicands
   const double inf = INFINITY, tiny = from_bits(1), least = from_bits(0x0010000000000000ULL);
