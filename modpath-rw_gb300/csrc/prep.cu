@@ -21,6 +21,24 @@
 
 namespace mprw {
 
+// Quotient and root on the integer pipe (fpbits.cuh: the operators' bits).  A
+// record takes some 170 quotients, of eight FP64 instructions each on a pipe
+// that holds a warp instruction for 16 clocks; out of line, since inlined they
+// would be most of the kernel's code.  Quotients by 1 (unit cells) and of
+// zeros are answered at once.  400,000 cells: 1.90 -> 0.68 ms.
+__device__ __noinline__ double quo(double a, double b) {
+  if (fb::is1(b)) return a;
+  if (fb::div_plain(a, b)) return fb::div_core(a, b, 0);
+  const unsigned eb = (unsigned)(fb::bits(b) >> 52) & 0x7FFu;
+  if (fb::is0(a) && eb - 1u < 2046u)
+    return fb::from_bits((fb::bits(a) ^ fb::bits(b)) & 0x8000000000000000ULL);
+  return a / b;
+}
+__device__ __noinline__ double root(double x) {
+  if (fb::sqrt_plain(x)) return fb::sqrt_core(x);
+  return sqrt(x);
+}
+
 __device__ __forceinline__ void klj(const GridDims &g, int n, int &k, int &i, int &j) {
   k = n / g.ncpl;
   int r = n - k * g.ncpl;
@@ -145,13 +163,13 @@ __device__ __forceinline__ void divergence_coeffs(const double A[8], const doubl
   monomials(A, a);
   monomials(B, b);
   monomials(C, c);
-  out[0] = (a[1] / DX + b[2] / DY + c[3] / DZ) * scale;
-  out[1] = (b[4] / DY + c[5] / DZ) * scale;  // x
-  out[2] = (a[4] / DX + c[6] / DZ) * scale;  // y
-  out[3] = (a[5] / DX + b[6] / DY) * scale;  // z
-  out[4] = (c[7] / DZ) * scale;              // xy
-  out[5] = (b[7] / DY) * scale;              // xz
-  out[6] = (a[7] / DX) * scale;              // yz
+  out[0] = (quo(a[1], DX) + quo(b[2], DY) + quo(c[3], DZ)) * scale;
+  out[1] = (quo(b[4], DY) + quo(c[5], DZ)) * scale;  // x
+  out[2] = (quo(a[4], DX) + quo(c[6], DZ)) * scale;  // y
+  out[3] = (quo(a[5], DX) + quo(b[6], DY)) * scale;  // z
+  out[4] = quo(c[7], DZ) * scale;                    // xy
+  out[5] = quo(b[7], DY) * scale;                    // xz
+  out[6] = quo(a[7], DX) * scale;                    // yz
 }
 
 // corner-component neighbour tables (TrackSubCell.F90:4142-4224, 4329-4363), 1-based
@@ -167,6 +185,8 @@ __constant__ int8_t kCPI[8][6] = {{1, 2, 7, 8, 13, 14},   {4, 5, 7, 8, 13, 15}, 
 // second-level neighbours of the six direct neighbours (ParticleTrackingEngine.f90:2033-2115)
 __constant__ int8_t kSub[6][2] = {{2, 3}, {2, 3}, {4, 5}, {4, 5}, {0, 1}, {0, 1}};
 
+constexpr int kRecThreads = 64;
+
 template <typename R>
 __device__ void store_record(CellRec<R> *dst, const double v1[3], const double v2[3], const double d[3],
                              const double div[3][7], const double vb[3][8], double aL, double aT, double aLV,
@@ -177,7 +197,7 @@ __device__ void store_record(CellRec<R> *dst, const double v1[3], const double v
     r.v1[m] = (R)v1[m];
     r.dv[m] = (R)(v2[m] - v1[m]);
     r.d[m] = (R)d[m];
-    r.inv_d[m] = (R)(1.0 / d[m]);
+    r.inv_d[m] = (R)quo(1.0, d[m]);
     r.v2[m] = (R)v2[m];
     for (int q = 0; q < 7; ++q) r.div[m][q] = (R)div[m][q];
     for (int q = 0; q < 8; ++q) r.vb[m][q] = (R)vb[m][q];
@@ -189,21 +209,22 @@ __device__ void store_record(CellRec<R> *dst, const double v1[3], const double v
   r.dm = (R)dm;
   r.two_over_r = (R)tr;
   r.dtcell = dtcell;
-  r.sqrt_dtcell = sqrt(dtcell);
+  r.sqrt_dtcell = root(dtcell);
   for (int f = 0; f < 6; ++f) r.conn[f] = conn[f];
   r.entry_status = es;
   r.massb = mb;
   *dst = r;
 }
 
-__global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *massb, CellRec<double> *rec64,
+// (16 warps per SM in 128 registers; 8 in 188 took 0.88 ms for the 400,000 cells)
+__global__ void __launch_bounds__(kRecThreads, 8) prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *massb, CellRec<double> *rec64,
                                 CellRec<float> *rec32) {
   const GridDims g = in.g;
   int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= g.ncell) return;
   int k, i, j;
   klj(g, n, k, i, j);
-  const double DX = in.delr[j] / 1.0, DY = in.delc[i] / 1.0, DZ = base.dz[n];
+  const double DX = in.delr[j], DY = in.delc[i], DZ = base.dz[n];
   const double phi = in.porosity[n], R = in.retardation[n];
   const double *Q = base.q + 6 * (int64_t)n;
   const uint8_t fl = base.flags[n];
@@ -212,12 +233,8 @@ __global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *mas
   if (in.backward) sign = -sign;
   // FillMassSubCellDataBuffer face velocities (ModpathCellData.f90:2559-2564)
   double v[6];
-  v[0] = sign * Q[0] / DY / DZ / phi / R;
-  v[1] = sign * Q[1] / DY / DZ / phi / R;
-  v[2] = sign * Q[2] / DX / DZ / phi / R;
-  v[3] = sign * Q[3] / DX / DZ / phi / R;
-  v[4] = sign * Q[4] / DX / DY / phi / R;
-  v[5] = sign * Q[5] / DX / DY / phi / R;
+  for (int f = 0; f < 6; ++f)
+    v[f] = quo(quo(quo(quo(sign * Q[f], f < 2 ? DY : DX), f < 4 ? DZ : DY), phi), R);
   int di = in.uniform_dispersion ? 0 : n;
   double aL = in.alpha_l[di], aT = in.alpha_t[di], dm = in.dm_eff[di];
   double aLV = in.alpha_lv ? in.alpha_lv[di] : aL, aTV = in.alpha_tv ? in.alpha_tv[di] : aT;
@@ -225,11 +242,11 @@ __global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *mas
   double mx = fmax(fabs(v[0]), fabs(v[1])), my = fmax(fabs(v[2]), fabs(v[3])), mz = fmax(fabs(v[4]), fabs(v[5]));
   double dtcell = 0.0;
   {
-    double adv = in.ts_param0 / (mx / DX + my / DY + mz / DZ);
-    double dsp = in.ts_param1 / (aL * mx / (DX * DX) + aT * my / (DY * DY) + aT * mz / (DZ * DZ));
+    double adv = quo(in.ts_param0, quo(mx, DX) + quo(my, DY) + quo(mz, DZ));
+    double dsp = quo(in.ts_param1, quo(aL * mx, DX * DX) + quo(aT * my, DY * DY) + quo(aT * mz, DZ * DZ));
     switch (in.time_step_kind) {
       case 1: dtcell = adv; break;
-      case 2: dtcell = in.ts_param1 / (aL * mx / (DX * DX) + aT * my / (DY * DY) + aT * mz / (DZ * DZ)); break;
+      case 2: dtcell = dsp; break;
       case 3: {
         double t = DBL_MAX;
         if (adv > 0.0 && adv < t) t = adv;
@@ -275,22 +292,22 @@ __global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *mas
       sa = sa + narea[kCXI[c][m] - 1][0];
       sf = sf + nflow(kCXI[c][m], kCXI[c][3]);
     }
-    qc[c][0] = sf / sa;
+    qc[c][0] = quo(sf, sa);
     sa = DX * DZ;
     sf = Q[kCYI[c][3] - 1];
     for (int m = 0; m < 3; ++m) {
       sa = sa + narea[kCYI[c][m] - 1][1];
       sf = sf + nflow(kCYI[c][m], kCYI[c][3]);
     }
-    qc[c][1] = sf / sa;
+    qc[c][1] = quo(sf, sa);
     sa = DX * DY;
     sf = Q[kCZI[c][3] - 1];
     for (int m = 0; m < 3; ++m) {
       sa = sa + narea[kCZI[c][m] - 1][2];
       sf = sf + nflow(kCZI[c][m], kCZI[c][3]);
     }
-    qc[c][2] = sf / sa;
-    qc[c][3] = sqrt(qc[c][0] * qc[c][0] + qc[c][1] * qc[c][1] + qc[c][2] * qc[c][2]);
+    qc[c][2] = quo(sf, sa);
+    qc[c][3] = root(qc[c][0] * qc[c][0] + qc[c][1] * qc[c][1] + qc[c][2] * qc[c][2]);
   }
   double phic[8];
   for (int c = 0; c < 8; ++c) {
@@ -303,7 +320,7 @@ __global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *mas
         sv = sv + nvol[q];
         sw = sw + nvol[q] * nphi[q];
       }
-      phic[c] = sw / sv;
+      phic[c] = quo(sw, sv);
     }
   }
   // qprod and isotropic corner dispersion (quirk: corners 3..8 use |q| of corner 100)
@@ -319,16 +336,16 @@ __global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *mas
       qp[4] = qc[c][1] * qc[c][2];
       qp[5] = qc[c][2] * qc[c][2];
       qp[6] = qp[0] + qp[3];
-      for (int m = 0; m < 7; ++m) qp[m] = qp[m] / qc[c][3];
+      for (int m = 0; m < 7; ++m) qp[m] = quo(qp[m], qc[c][3]);
     }
     if (in.dispersion_model == 1) {
       // pr_CornerDispersionAxisymmetric (TrackSubCell.F90:3117-3303): per
       // corner alphaL/alphaT blended with cosinesq = qz**2/|q| (as written),
       // Dxyx from the xx product (as written)
-      if (qc[c][3] > 0.0 && qp[6] > 0.0) qp[7] = (qc[c][2] * qc[c][2]) / (qc[c][0] * qc[c][0] + qc[c][1] * qc[c][1]);
+      if (qc[c][3] > 0.0 && qp[6] > 0.0) qp[7] = quo(qc[c][2] * qc[c][2], qc[c][0] * qc[c][0] + qc[c][1] * qc[c][1]);
       const double pD = phic[c] * dm;
       double cosinesq = 0.0;
-      if (qc[c][3] > 0.0) cosinesq = qc[c][2] * qc[c][2] / qc[c][3];
+      if (qc[c][3] > 0.0) cosinesq = quo(qc[c][2] * qc[c][2], qc[c][3]);
       const double aLc = aL + cosinesq * (aLV - aL);
       const double aTc = aTV + cosinesq * (aT - aTV);
       const double aLmTc = aLc - aTc;
@@ -356,7 +373,7 @@ __global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *mas
     D[8][c] = D[6][c];
   }
   // divergence coefficients, (sum)/porosity/retardation folded into one scale
-  double scale = 1.0 / (phi * R);
+  double scale = quo(1.0, phi * R);
   double div[3][7];
   divergence_coeffs(D[0], D[5], D[7], DX, DY, DZ, scale, div[0]);  // Dxxx, Dxyy, Dxzz
   divergence_coeffs(D[3], D[1], D[8], DX, DY, DZ, scale, div[1]);  // Dxyx, Dyyy, Dyzz
@@ -365,7 +382,7 @@ __global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *mas
   double vb[3][8];
   for (int m = 0; m < 3; ++m) {
     double cv[8];
-    for (int c = 0; c < 8; ++c) cv[c] = qc[c][m] / phic[c];
+    for (int c = 0; c < 8; ++c) cv[c] = quo(qc[c][m], phic[c]);
     monomials(cv, vb[m]);
   }
   // entry checks
@@ -405,7 +422,7 @@ __global__ void prep_rec_kernel(PrepInputs in, CellBase base, const uint8_t *mas
     conn[f] = (m >= 0 && in.iboundts[m] != 0) ? m : -1;
   }
   double v1[3] = {v[0], v[2], v[4]}, v2[3] = {v[1], v[3], v[5]}, d[3] = {DX, DY, DZ};
-  double tr = 2.0 / R;
+  double tr = quo(2.0, R);
   if (rec64)
     store_record<double>(rec64 + n, v1, v2, d, div, vb, aL, aT, aLV, aTV, dm, tr, dtcell, conn, es, massb[n]);
   if (rec32)
@@ -419,7 +436,7 @@ cudaError_t launch_prep(const PrepInputs &in, CellBase base, uint8_t *massb, Cel
   prep_base_kernel<<<blocks, threads, 0, s>>>(in, base, massb);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  prep_rec_kernel<<<blocks, threads, 0, s>>>(in, base, massb, rec64, rec32);
+  prep_rec_kernel<<<(in.g.ncell + kRecThreads - 1) / kRecThreads, kRecThreads, 0, s>>>(in, base, massb, rec64, rec32);
   return cudaGetLastError();
 }
 
