@@ -64,6 +64,10 @@ struct PrepInputs {
   int32_t backward, stop_weak_sinks, stop_weak_sources, stop_zone, uniform_porosity;
 };
 
+// what a flow time step's check found (bits of *flag)
+enum : int { FLOW_BAD_POROSITY = 1, FLOW_NON_FINITE = 2, FLOW_NAN_HEAD = 4, FLOW_BAD_JA = 8 };
+cudaError_t launch_flow_check(const PrepInputs &in, int64_t nja, int64_t ndisp, int *flag, cudaStream_t s);
+cudaError_t launch_sattop(const PrepInputs &in, double *sattop, cudaStream_t s);
 cudaError_t launch_prep(const PrepInputs &in, CellBase base, uint8_t *massb, CellRec<double> *rec64,
                         CellRec<float> *rec32, cudaStream_t s);
 

@@ -429,6 +429,66 @@ __global__ void __launch_bounds__(kRecThreads, 8) prep_rec_kernel(PrepInputs in,
     store_record<float>(rec32 + n, v1, v2, d, div, vb, aL, aT, aLV, aTV, dm, tr, dtcell, conn, es, massb[n]);
 }
 
+// The checks a load makes before anything uses its arrays, in one pass over
+// them (bandwidth; the host took 4 ms over the same arrays).
+__device__ __forceinline__ bool finite_bits(double v) {
+  return (fb::bits(v) & 0x7FF0000000000000ULL) != 0x7FF0000000000000ULL;
+}
+__global__ void flow_check_kernel(PrepInputs in, int64_t nja, int64_t ndisp, int *flag) {
+  const int64_t nc = in.g.ncell, i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  int bad = 0;
+  auto all_finite = [&](const double *a, int64_t n) {
+    if (!a) return;
+    for (int64_t i = i0; i < n; i += step)
+      if (!finite_bits(a[i])) bad |= FLOW_NON_FINITE;
+  };
+  for (int64_t i = i0; i < nja; i += step) {
+    const int32_t m = in.ja[i];
+    if (m < 1 || m > nc) bad |= FLOW_BAD_JA;
+  }
+  all_finite(in.flowja, nja);
+  all_finite(in.bflow, 6 * nc);
+  all_finite(in.source_flow, nc);
+  all_finite(in.sink_flow, nc);
+  all_finite(in.alpha_l, ndisp);
+  all_finite(in.alpha_t, ndisp);
+  all_finite(in.dm_eff, ndisp);
+  all_finite(in.alpha_lv, ndisp);
+  all_finite(in.alpha_tv, ndisp);
+  for (int64_t i = i0; i < nc; i += step) {
+    const double p = in.porosity[i], r = in.retardation[i];
+    if (!fb::above0(p) || !fb::above0(r) || !finite_bits(p) || !finite_bits(r)) bad |= FLOW_BAD_POROSITY;
+    if (in.heads && fb::isnan_bits(in.heads[i])) bad |= FLOW_NAN_HEAD;
+  }
+  bad = __reduce_or_sync(0xffffffffu, (unsigned)bad);
+  if (bad && (threadIdx.x & 31) == 0) atomicOr(flag, bad);
+}
+
+cudaError_t launch_flow_check(const PrepInputs &in, int64_t nja, int64_t ndisp, int *flag, cudaStream_t s) {
+  const int64_t b = (nja + 255) / 256;
+  flow_check_kernel<<<(int)(b < 152 * 8 ? b : 152 * 8), 256, 0, s>>>(in, nja, ndisp, flag);
+  return cudaGetLastError();
+}
+
+// SaturatedTop of every cell (FlowModelData.f90:258-279): the head of an
+// active convertible cell that holds it, else the cell's top
+__global__ void sattop_kernel(PrepInputs in, double *sattop) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= in.g.ncell) return;
+  double t = n < in.g.ncpl ? in.top[n] : in.botm[n - in.g.ncpl];
+  if (in.celltype && in.heads && in.celltype[n] == 1 && in.iboundts[n] != 0) {
+    const double hd = in.heads[n];
+    if (hd <= t && hd >= in.botm[n]) t = hd;
+  }
+  sattop[n] = t;
+}
+
+cudaError_t launch_sattop(const PrepInputs &in, double *sattop, cudaStream_t s) {
+  sattop_kernel<<<(in.g.ncell + 255) / 256, 256, 0, s>>>(in, sattop);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_prep(const PrepInputs &in, CellBase base, uint8_t *massb, CellRec<double> *rec64,
                         CellRec<float> *rec32, cudaStream_t s) {
   int threads = 128;
