@@ -1,0 +1,48 @@
+"""The density scatter and the gathers at the grid shapes where their loops
+turn over: spans of one cell, of a few, of more than a warp (32) and of more
+layers than the row cache takes at once; grids narrower than the kernels
+(windows folded at both edges), odd sizes, one, two and three dimensions.
+FP64 against the numpy restatement on the same particles (1e-9 of the
+largest density and the same number of loops, as test_gpu_gpkde), FP32
+against FP64 (1e-3 of the largest density, as there)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+import mprw
+from mprw import workloads as W
+from mprw.model import ACTIVE, MIXED
+from oracle import gpkde_oracle as GO
+
+# (ncol, nrow, nlay), bin size along x, particles
+SHAPES = [
+    ((97, 1, 1), 1.0, 700),
+    ((33, 7, 3), 1.0, 500),
+    ((5, 3, 2), 1.0, 400),
+    ((12, 10, 40), 1.0, 900),
+    ((70, 5, 9), 0.5, 800),
+]
+
+
+@pytest.mark.parametrize("dims,bin_x,n", SHAPES)
+def test_reconstruction_at_the_edges_of_the_loops(gpu_lib, dims, bin_x, n):
+    ncol, nrow, nlay = dims
+    g, f, p, opt, _ = W.lognormal_slab(n_particles=n, nlay=nlay, nrow=nrow, ncol=ncol, seed=4, use_torch=False)
+    dom, bins = (float(ncol), float(nrow), float(nlay)), (bin_x, 1.0, 1.0)
+    tr = mprw.Tracker(g, opt)
+    tr.load_flow(f)
+    tr.set_particles(p)
+    tr.advance(0.0, 0.5)
+    out = tr.get_particles()
+    act = out["status"] == ACTIVE
+    co = np.stack([out["gx"], out["gy"], out["gz"]], 1)[act]
+    assert co.shape[0] >= 50  # particles left in the grid
+    dens, hist, loops = tr.gpkde(dom, bins, n_opt_loops=3)
+    d32, _, _ = tr.gpkde(dom, bins, n_opt_loops=3, precision=MIXED)
+    tr.close()
+    G = GO.GPKDE(dom, bins, n_opt_loops=3)
+    ref, _ = G.compute_density(co, np.ones(co.shape[0]))
+    assert loops == G.loops
+    np.testing.assert_allclose(dens, ref.transpose(2, 1, 0), rtol=0, atol=1e-9 * ref.max())
+    np.testing.assert_allclose(d32, dens, rtol=0, atol=1e-3 * dens.max())
