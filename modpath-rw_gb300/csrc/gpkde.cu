@@ -62,6 +62,7 @@ __device__ __forceinline__ float root(float x) { return sqrtf(x); }
 
 constexpr int kThreads = 256;
 constexpr int kBinThreads = 64;   // per-bin elementwise kernels: spread few bins over all SMs
+constexpr int kMaskedBins = 16384;
 constexpr int kPassBlocks = 2432; // most blocks of a separable pass: 16 per SM (measured best of 4-48), grid-stride over all keys' regions
 
 // The database level of a kernel size h along dimension d:
@@ -789,42 +790,39 @@ __global__ void gather_x_kernel(KdeParams P, const SepPlan *pl, const T *val, Fi
 // the plume, while the z pass reads pass 2 only at the bins' columns within
 // mz of the bins (their z windows, folded or not, stay inside them) and the
 // y pass reads pass 1 only within my of those elements.  mark_needed_kernel
-// and dilate_needed_kernel flag these elements (byte masks over the pass
-// buffers' layout), and the masked passes compute only them: each warp
-// gathers the flagged elements of its chunks into a shared queue and runs
-// them 32 at a time, so the FP64 multiply-adds run on full warps.  Elements
-// left unflagged are never read.  On the bench workload the flagged
-// elements are ~30 % of pass 1's and ~17 % of pass 2's.
+// and list_needed_kernel flag these elements (byte masks over the pass
+// buffers' layout) and list them, runs of the buffer's order one after the
+// other, and the passes run down the lists; elements left unflagged are never
+// read.  At 1,000,000 particles on 200 x 100 x 20 bins they are ~30 % of pass
+// 1's and ~17 % of pass 2's elements.  A list's neighbours share a key, so a
+// warp's windows are equally long and its FP64 multiply-adds run on full
+// warps, and the lists divide evenly over the grid.  (Warps that scanned the
+// masks and queued what they found mixed keys, and their shares differed: x
+// passes 1.56 -> 0.98 ms per reconstruction, y passes 1.19 -> 0.69, the lists
+// 0.10; the multiply-adds bound them now.)  The order of the lists varies from
+// run to run; no element's value depends on it.
+//
+// A list holds a quarter of its buffer's elements.  Six fields per element
+// take six times the space, so that is enough for every plan of theirs; a plan
+// that flags more scans the mask instead.
 template <typename F>
-__device__ __forceinline__ void for_needed(long long tot, const unsigned char *mask, int (*q)[64], F &&visit) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  int cnt = 0;
-  for (long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + w) * 32; base < tot; base += nwarps * 32) {
-    const long long e = base + lane;
-    const bool need = e < tot && mask[e] != 0;
-    const unsigned bal = __ballot_sync(0xffffffffu, need);
-    if (need) q[w][cnt + __popc(bal & ((1u << lane) - 1u))] = (int)e;
-    cnt += __popc(bal);
-    __syncwarp();
-    if (cnt >= 32) {
-      visit((long long)q[w][lane]);
-      __syncwarp();
-      if (lane < cnt - 32) q[w][lane] = q[w][lane + 32];
-      cnt -= 32;
-      __syncwarp();
-    }
+__device__ __forceinline__ void for_needed(long long tot, const unsigned char *mask, const int *list, long long n,
+                                           long long cap, F &&visit) {
+  const bool listed = n <= cap;
+  const long long end = listed ? n : tot;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < end; i += (long long)gridDim.x * blockDim.x) {
+    const long long g = listed ? (long long)list[i] : i;
+    if (listed || mask[g] != 0) visit(g);
   }
-  if (lane < cnt) visit((long long)q[w][lane]);
 }
 
 template <typename T, int NC>
 __global__ void __launch_bounds__(kThreads) gather_x_masked_kernel(KdeParams P, const SepPlan *pl, const T *val,
-                                                                  Fields<T> F, const unsigned char *mask, T *T1) {
+                                                                  Fields<T> F, const unsigned char *mask,
+                                                                  const int *list, long long cap, T *T1) {
   __shared__ long long so[KDE_KMAX];
-  __shared__ int q[kThreads / 32][64];
   const int np = load_offsets(pl, pl->o1, so);
-  for_needed(pl->tot1, mask, q, [&](long long g) { gx_element<T, NC>(P, pl, val, F, T1, so, np, g); });
+  for_needed(pl->tot1, mask, list, pl->n1, cap, [&](long long g) { gx_element<T, NC>(P, pl, val, F, T1, so, np, g); });
 }
 
 // flag pass 2's elements at the bins' columns within mz of each bin
@@ -841,30 +839,71 @@ __global__ void mark_needed_kernel(KdeBinsT<T> B, const SepPlan *pl, const int *
   }
 }
 
-// flag pass 1's elements within my of every flagged element of pass 2
-__global__ void dilate_needed_kernel(const SepPlan *pl, const unsigned char *m2, unsigned char *m1) {
+// List the flagged elements of one pass, 1,024 of its buffer per block and
+// turn: four flags per thread, a block-wide count, one reservation (2,048
+// left pass 2's blocks too unequal, 512 cost pass 1 more than they gave).  Pass 2's
+// (DILATE) also flag pass 1's elements within my of each: with the element
+// before it along y flagged too, all but the last of these are that one's.
+constexpr int kListBytes = 4;
+template <bool DILATE>
+__global__ void __launch_bounds__(kThreads) list_needed_kernel(SepPlan *pl, const unsigned char *m, unsigned char *m1,
+                                                              int *list, long long cap) {
   __shared__ long long so[KDE_KMAX];
+  __shared__ int item[kThreads * kListBytes], wsum[kThreads / 32];
+  __shared__ long long first;
   const int np = load_offsets(pl, pl->o2, so);
-  const long long tot = pl->tot2;
-  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < tot; g += (long long)gridDim.x * blockDim.x) {
-    if (!m2[g]) continue;
-    const int j = flat_slot(so, np, g);
-    const int *r1 = pl->r1[j], *r2 = pl->r2[j];
-    int x, y, z;
-    region_xyz(r2, g - so[j], x, y, z);
-    const int my = pl->m[j][1];
-    const int y0 = max(r1[2], y - my), y1 = min(r1[3], y + my);
-    unsigned char *m = m1 + pl->o1[j];
-    for (int yy = y0; yy <= y1; ++yy) m[region_loc(r1, x, yy, z)] = 1;
+  const long long tot = DILATE ? pl->tot2 : pl->tot1;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (long long b = blockIdx.x * (long long)(kThreads * kListBytes); b < tot; b += (long long)gridDim.x * (kThreads * kListBytes)) {
+    const long long e = b + threadIdx.x * kListBytes;
+    // (the masks are cleared to the next eight)
+    const unsigned v = e < tot ? *reinterpret_cast<const unsigned *>(m + e) : 0u;
+    const int c = __popc(v);
+    int s = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += t;
+    }
+    if (lane == 31) wsum[w] = s;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int i = 0; i < kThreads / 32; ++i) {
+      if (i < w) before += wsum[i];
+      total += wsum[i];
+    }
+    int o = before + s - c;
+    for (int k = 0; k < kListBytes; ++k)
+      if ((v >> (8 * k)) & 1) item[o++] = (int)(e + k);
+    if (threadIdx.x == 0 && total)
+      first = (long long)atomicAdd(DILATE ? &pl->n2 : &pl->n1, (unsigned long long)total);
+    __syncthreads();
+    for (int i = threadIdx.x; i < total; i += kThreads) {
+      const int g = item[i];
+      if (first + i < cap) list[first + i] = g;
+      if constexpr (DILATE) {
+        const int j = flat_slot(so, np, g);
+        const int *r1 = pl->r1[j], *r2 = pl->r2[j];
+        int x, y, z;
+        region_xyz(r2, g - so[j], x, y, z);
+        const int my = pl->m[j][1];
+        const bool prev = y > r2[2] && m[g - (r2[1] - r2[0] + 1)] != 0;
+        const int y0 = max(r1[2], prev ? y + my : y - my), y1 = min(r1[3], y + my);
+        unsigned char *q = m1 + pl->o1[j];
+        for (int yy = y0; yy <= y1; ++yy) q[region_loc(r1, x, yy, z)] = 1;
+      }
+    }
+    __syncthreads();
   }
 }
 
-__global__ void clear_needed_kernel(const SepPlan *pl, unsigned char *m1, unsigned char *m2) {
-  const long long t1 = pl->tot1, t2 = pl->tot2;
-  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < t1 || g < t2;
+__global__ void clear_needed_kernel(SepPlan *pl, unsigned char *m1, unsigned char *m2) {
+  const long long w1 = (pl->tot1 + 7) / 8, w2 = (pl->tot2 + 7) / 8;
+  if (blockIdx.x == 0 && threadIdx.x == 0) pl->n1 = pl->n2 = 0;
+  unsigned long long *q1 = reinterpret_cast<unsigned long long *>(m1), *q2 = reinterpret_cast<unsigned long long *>(m2);
+  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < w1 || g < w2;
        g += (long long)gridDim.x * blockDim.x) {
-    if (g < t1) m1[g] = 0;
-    if (g < t2) m2[g] = 0;
+    if (g < w1) q1[g] = 0;
+    if (g < w2) q2[g] = 0;
   }
 }
 
@@ -970,11 +1009,11 @@ __global__ void gather_y_kernel(KdeParams P, const SepPlan *pl, const T *val, co
 
 template <typename T, int NC>
 __global__ void __launch_bounds__(kThreads) gather_y_masked_kernel(KdeParams P, const SepPlan *pl, const T *val,
-                                                                  const T *T1, const unsigned char *mask, T *T2) {
+                                                                  const T *T1, const unsigned char *mask,
+                                                                  const int *list, long long cap, T *T2) {
   __shared__ long long so[KDE_KMAX];
-  __shared__ int q[kThreads / 32][64];
   const int np = load_offsets(pl, pl->o2, so);
-  for_needed(pl->tot2, mask, q, [&](long long g) { gy_element<T, NC>(P, pl, val, T1, T2, so, np, g); });
+  for_needed(pl->tot2, mask, list, pl->n2, cap, [&](long long g) { gy_element<T, NC>(P, pl, val, T1, T2, so, np, g); });
 }
 
 // Gather pass 3 at every bin: sum_t fz[t] T2(bx, by, reflect(bz - m + t)).
@@ -1635,30 +1674,45 @@ cudaError_t KdeState::ensure_grid(int64_t ngrid) {
   return cudaSuccess;
 }
 
+// a list of needed elements: the passes do without (they scan the masks)
+// where the memory does not reach
+static int64_t alloc_list(int **p, int64_t n) {
+  if (cudaMalloc((void **)p, sizeof(int) * n) == cudaSuccess) return n;
+  (void)cudaGetLastError();
+  *p = nullptr;
+  return 0;
+}
+
 cudaError_t KdeState::ensure_pass(int64_t n1, int64_t n2) {
   if (n1 > t1_cap) {
     if (t1) cudaFree(t1);
     if (need1) cudaFree(need1);
+    if (list1) cudaFree(list1);
     t1 = nullptr;
     need1 = nullptr;
-    t1_cap = 0;
+    list1 = nullptr;
+    t1_cap = list1_cap = 0;
     const int64_t c = n1 + n1 / 4;
     cudaError_t e = cudaMalloc((void **)&t1, sizeof(double) * c);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&need1, c);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&need1, c + 8);
     if (e != cudaSuccess) return e;
     t1_cap = c;
+    list1_cap = alloc_list(&list1, c / 4);
   }
   if (n2 > t2_cap) {
     if (t2) cudaFree(t2);
     if (need2) cudaFree(need2);
+    if (list2) cudaFree(list2);
     t2 = nullptr;
     need2 = nullptr;
-    t2_cap = 0;
+    list2 = nullptr;
+    t2_cap = list2_cap = 0;
     const int64_t c = n2 + n2 / 4;
     cudaError_t e = cudaMalloc((void **)&t2, sizeof(double) * c);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&need2, c);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&need2, c + 8);
     if (e != cudaSuccess) return e;
     t2_cap = c;
+    list2_cap = alloc_list(&list2, c / 4);
   }
   return cudaSuccess;
 }
@@ -1667,7 +1721,7 @@ void KdeState::release() {
   void *ptrs[] = {bins.gx, bins.gy, bins.gz, bins.count, bins.ks, bins.scale, bins.shape, bins.support, bins.nest,
                   bins.dens, bins.cb, bins.rxx, bins.ryy, bins.rzz, bins.net, bins.dens_old, bins.scale_old,
                   partial, dens_grid, cx, cy, cz, d_scalars, d_flag, d_blockcnt, d_val, d_valf, d_meta, cell_bin,
-                  bin_key, d_keys, d_plan, t1, t2, need1, need2, d_wcnt, dens_raw, d_need, cxy, cxz, cyz, dens_out};
+                  bin_key, d_keys, d_plan, t1, t2, need1, need2, list1, list2, d_wcnt, dens_raw, d_need, cxy, cxz, cyz, dens_out};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (h_scalars) cudaFreeHost(h_scalars);
@@ -1950,23 +2004,30 @@ static cudaError_t kde_attempt(KdeState &st, const KdeParams &P, double hs, doub
     st.launches += 1;
     return cudaGetLastError();
   };
-  // FP64: the gathers compute only the pass elements that are read (the
-  // masks follow each smoothing-kernel plan); their element numbers must fit
-  // an int (the pass capacity bounds them)
-  const bool masked = sizeof(T) == 8 && st.t1_cap < (int64_t)INT_MAX && st.t2_cap < (int64_t)INT_MAX;
+  // FP64: the gathers compute only the pass elements that are read (masks and
+  // lists follow each smoothing-kernel plan); their element numbers must fit
+  // an int (the pass capacity bounds them).  From 16,384 active bins: below,
+  // the four launches that find the elements take longer than the elements
+  // left out (ms per reconstruction of 8 loops without and with them: 3,171
+  // bins 1.66 and 1.90, 6,607 1.90 and 2.10, 11,200 2.24 and 2.40, 24,191 3.42
+  // and 3.25, 56,392 7.38 and 6.15).  FP32's multiply-adds cost a sixteenth
+  // and the launches as much: with lists 300,000 particles on 187 x 93 x 21
+  // bins took 3.90 ms for 3.80.
+  const bool masked = sizeof(T) == 8 && nb >= kMaskedBins && st.t1_cap < (int64_t)INT_MAX && st.t2_cap < (int64_t)INT_MAX;
   auto needed = [&](void) -> cudaError_t {
     if (!masked) return cudaSuccess;
     clear_needed_kernel<<<pgrid, kThreads, 0, s>>>(plan1, st.need1, st.need2);
     mark_needed_kernel<T><<<bb, kBinThreads, 0, s>>>(B, plan1, key1, st.need2);
-    dilate_needed_kernel<<<pgrid, kThreads, 0, s>>>(plan1, st.need2, st.need1);
-    st.launches += 3;
+    list_needed_kernel<true><<<pgrid, kThreads, 0, s>>>(plan1, st.need2, st.need1, st.list2, st.list2_cap);
+    list_needed_kernel<false><<<pgrid, kThreads, 0, s>>>(plan1, st.need1, nullptr, st.list1, st.list1_cap);
+    st.launches += 4;
     return cudaGetLastError();
   };
   auto gather_xy = [&](auto nc_tag, Fields<T> F) -> cudaError_t {
     constexpr int NC = decltype(nc_tag)::value;
     if (masked) {
-      gather_x_masked_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, F, st.need1, t1);
-      gather_y_masked_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, t1, st.need2, t2);
+      gather_x_masked_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, F, st.need1, st.list1, st.list1_cap, t1);
+      gather_y_masked_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, t1, st.need2, st.list2, st.list2_cap, t2);
     } else {
       gather_x_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, F, t1);
       gather_y_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, t1, t2);

@@ -63,6 +63,7 @@ struct KeyAcc {
 // intermediate passes and their offsets (in elements) into the pass buffers.
 struct SepPlan {
   int np;
+  unsigned long long n1, n2;  // needed elements (FP64 gathers)
   long long tot1, tot2;  // elements (region cells) of the two pass buffers, all keys
   int slot_of[KDE_KMAX];
   int key[KDE_KMAX];
@@ -102,7 +103,10 @@ struct KdeState {
   SepPlan *d_plan = nullptr;
   double *t1 = nullptr, *t2 = nullptr;
   int64_t t1_cap = 0, t2_cap = 0;
-  unsigned char *need1 = nullptr, *need2 = nullptr;  // FP64 gathers: the elements of the passes that are read
+  // FP64 gathers: the elements of the passes that are read, as masks and lists
+  unsigned char *need1 = nullptr, *need2 = nullptr;
+  int *list1 = nullptr, *list2 = nullptr;
+  int64_t list1_cap = 0, list2_cap = 0;
   double work_madds = 0;  // the last reconstruction's work model (multiply-adds of direct kernels)
   // run the optimisation loop as a device-side graph loop when the stream can
   // be captured; a batch's workers drive it from the host (several small

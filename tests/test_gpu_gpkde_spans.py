@@ -46,3 +46,28 @@ def test_reconstruction_at_the_edges_of_the_loops(gpu_lib, dims, bin_x, n):
     assert loops == G.loops
     np.testing.assert_allclose(dens, ref.transpose(2, 1, 0), rtol=0, atol=1e-9 * ref.max())
     np.testing.assert_allclose(d32, dens, rtol=0, atol=1e-3 * dens.max())
+
+
+@pytest.mark.parametrize("dims,n", [((61, 37, 9), 150_000), ((31, 29, 17), 20_000), ((523, 40, 1), 120_000)])
+def test_needed_elements_of_the_gathers(gpu_lib, dims, n):
+    """FP64 gathers over the elements that are read: more active bins than the
+    16,384 from which the passes run down lists of them (and fewer, where
+    they do not), plumes over odd grids whose windows fold at every face."""
+    ncol, nrow, nlay = dims
+    g, f, p, opt, _ = W.lognormal_slab(n_particles=8, nlay=nlay, nrow=nrow, ncol=ncol, seed=5, use_torch=False)
+    p = W.release_in_box(g, n, 0.0, float(ncol), 0.0, float(nrow), float(g.botm[-1]), float(g.top[0]), seed=6)
+    dom, bins = (float(ncol), float(nrow), float(nlay)), (1.0, 1.0, 1.0)
+    tr = mprw.Tracker(g, opt)
+    tr.load_flow(f)
+    tr.set_particles(p)
+    tr.advance(0.0, 0.01)
+    out = tr.get_particles()
+    act = out["status"] == ACTIVE
+    co = np.stack([out["gx"], out["gy"], out["gz"]], 1)[act]
+    dens, hist, loops = tr.gpkde(dom, bins, n_opt_loops=1)
+    tr.close()
+    assert ((hist > 0).sum() >= 16384) == (n > 100_000)
+    G = GO.GPKDE(dom, bins, n_opt_loops=1)
+    ref, _ = G.compute_density(co, np.ones(co.shape[0]))
+    assert loops == G.loops
+    np.testing.assert_allclose(dens, ref.transpose(2, 1, 0), rtol=0, atol=1e-9 * ref.max())
