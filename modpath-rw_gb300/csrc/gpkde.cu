@@ -62,6 +62,7 @@ __device__ __forceinline__ float root(float x) { return sqrtf(x); }
 
 constexpr int kThreads = 256;
 constexpr int kBinThreads = 64;   // per-bin elementwise kernels: spread few bins over all SMs
+constexpr int kDeviceLoopBins = 8192;
 constexpr int kMaskedBins = 16384;
 constexpr int kPassBlocks = 2432; // most blocks of a separable pass: 16 per SM (measured best of 4-48), grid-stride over all keys' regions
 
@@ -2119,7 +2120,12 @@ static cudaError_t kde_attempt(KdeState &st, const KdeParams &P, double hs, doub
   st.launches += 2;
   KCK(density());
   KCK(reduce(RED_ALMISE));  // nEstimate and net roughness are zero: 0
-  if (n_opt_loops > 0 && st.device_loop) {
+  // A conditional graph takes some 0.25 ms to build, more than the host's read
+  // after each of the few loops a small reconstruction runs; the host-driven
+  // loop's graph is kept and updated.  (ms, device and host: 7 bins 0.53 and
+  // 0.47, 1,459 bins 2.00 and 1.98, 3,171 bins 1.66 and 1.65, 56,392 bins both
+  // 7.38 -- there the host's reads would only tie up its thread.)
+  if (n_opt_loops > 0 && st.device_loop && nb >= kDeviceLoopBins) {
     // the whole loop as one graph: a while node around the captured body (a
     // while node runs its body at least once: no loops are the host path's)
     cudaGraphExec_t dexec = nullptr;

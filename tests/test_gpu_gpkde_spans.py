@@ -71,3 +71,24 @@ def test_needed_elements_of_the_gathers(gpu_lib, dims, n):
     ref, _ = G.compute_density(co, np.ones(co.shape[0]))
     assert loops == G.loops
     np.testing.assert_allclose(dens, ref.transpose(2, 1, 0), rtol=0, atol=1e-9 * ref.max())
+
+
+def test_small_reconstruction_on_a_stream_and_on_the_default_stream(gpu_lib):
+    """Below the bins from which the loop runs on the device the host drives
+    it, as a kept graph on a stream that can be captured and launch by launch
+    on the legacy default stream: the same loops, the same bits, also for a
+    second reconstruction that finds the kept graph."""
+    g, f, p, opt = W.uniform_pulse(n_particles=5000)
+    tr = mprw.Tracker(g, opt)
+    tr.load_flow(f)
+    tr.set_particles(p)
+    for t0, t1 in ((0.0, 20.0), (20.0, 40.0)):
+        tr.advance(t0, t1)
+        d0, h0, l0 = tr.gpkde((200.0, 1.0, 1.0), (1.0, 1.0, 1.0))
+        tr.set_stream(1)  # cudaStreamLegacy
+        d1, h1, l1 = tr.gpkde((200.0, 1.0, 1.0), (1.0, 1.0, 1.0))
+        tr.set_stream(0)
+        assert l0 == l1 > 0
+        np.testing.assert_array_equal(h0, h1)
+        assert np.array_equal(d0.view(np.uint64), d1.view(np.uint64))
+    tr.close()
