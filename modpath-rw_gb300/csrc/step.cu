@@ -440,17 +440,27 @@ __device__ __forceinline__ bool quad_axis_f64(bool high, double pos, double d, d
 // Newton-Raphson (:1895-2554).  Both run in FP64 whatever the particle
 // precision: the displacement v (e^{dv dt} - 1)/dv and the exit-time solve
 // lose their digits to cancellation at small velocity gradients.
+// Their quotients and displacements are calls: inlined at some thirty sites the
+// integer divisions made the kernel's code longer than the instruction caches
+// hold, and with the few warps that this kernel runs a third of the time went
+// into fetching it (40,001 particles of a 61x37x7 field, two 5-day intervals,
+// 57 -> 43 ms; 200,001, one interval: 99 -> 64).
+__device__ __noinline__ double div_n(double a, double b) { return div_r(a, b); }
 // em1 = e^{dvdx dt} - 1
 __device__ __forceinline__ double adv_exponential(double v, double dvdx, double dt, double em1) {
   const double dvtol = 1.0e-10;
-  return lt_any(dvtol, fabs(dvdx)) ? div_r(v * em1, dvdx) : v * dt;
+  return lt_any(dvtol, fabs(dvdx)) ? div_n(v * em1, dvdx) : v * dt;
 }
 
-__device__ __forceinline__ double nr_conv_g(double f0, double f1, double f2) { return fabs(div_r(f2 * f0, f1 * f1)); }
+__device__ __noinline__ double exp_displacement(double v, double dvdx, double dt) {
+  return adv_exponential(v, dvdx, dt, exp(dvdx * dt) - 1.0);
+}
+
+__device__ __forceinline__ double nr_conv_g(double f0, double f1, double f2) { return fabs(div_n(f2 * f0, f1 * f1)); }
 __device__ __forceinline__ double nr_conv_gder(double f0, double f1, double f2, double f3) {
-  const double gna = div_r(f2 * f0, f1 * f1);
-  const double gpp = div_r(-2.0 * (f0 * (f2 * f2)), f1 * f1 * f1) + div_r(f1 * f2 + f0 * f3, f1 * f1);
-  return div_r(gna, fabs(gna)) * gpp;
+  const double gna = div_n(f2 * f0, f1 * f1);
+  const double gpp = div_n(-2.0 * (f0 * (f2 * f2)), f1 * f1 * f1) + div_n(f1 * f2 + f0 * f3, f1 * f1);
+  return div_n(gna, fabs(gna)) * gpp;
 }
 // |x| < 1, 1/2 for x = |..| (NaN: false, as the compare)
 __device__ __forceinline__ bool mag_below(double x, double c) { return fb::bits(x) < fb::bits(c); }
@@ -489,18 +499,18 @@ __device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, do
     if (!is0(at) || phase == NEWTON) {
       const double e = exp(dvdx * at), s = sqrt_r(at);
       f0 = adv_exponential(v, dvdx, at, e - 1.0) + divD * at + dB * s - dI;
-      const double q = div_r(dB, s);
+      const double q = div_n(dB, s);
       f1 = v * e + divD + 0.5 * q;
       if (phase != NEWTON) {
         ve = e;
         fat = at;
-        f2 = dvdx * v * e - 0.25 * div_r(q, at);
+        f2 = dvdx * v * e - 0.25 * div_n(q, at);
       }
     }
     bool guess = false;  // the initial guess is dtnew: go on to Newton
     bool derive = false;   // the guess goes on: a pass of its 50-pass loop
     if (phase == NEWTON) {
-      nrerror = div_r(-f0, f1);
+      nrerror = div_n(-f0, f1);
       dtnew = dtnew + nrerror;
       if (below0(dtnew)) dtnew = -(double)0.9f * dtnew;
       ++counter;
@@ -520,7 +530,7 @@ __device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, do
         }
         if (phase == SCAN2) {
           if (mag_below(gprimmin, 1.0)) dtnew = dt * mindtfrac;
-          if ((below0(dtnew) || is0(dtnew)) && above0(fabs(v))) dtnew = fabs(div_r(dI, v));
+          if ((below0(dtnew) || is0(dtnew)) && above0(fabs(v))) dtnew = fabs(div_n(dI, v));
           guess = true;
         } else {
           double dtoldfraction;
@@ -529,7 +539,7 @@ __device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, do
             dtoldfraction = kP10[gcount - 1];
           } else {
             dtfraction = mindtfrac;
-            dtoldfraction = div_r(0.5 * dtfraction, 10.0);
+            dtoldfraction = div_n(0.5 * dtfraction, 10.0);
           }
           dtnew = dtfraction * dt;
           dtold = dtoldfraction * dt;
@@ -553,7 +563,7 @@ __device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, do
       } else if (phase == ITER) {
         gprimnew = g;
         bool out = false;
-        if (mag_below(gprimnew, 1.0) && above0(dtnew) && mag_below(div_r(dtnew, dt), 1.0)) {
+        if (mag_below(gprimnew, 1.0) && above0(dtnew) && mag_below(div_n(dtnew, dt), 1.0)) {
           rcount = rcount + 1;
           guess = rcount > 1;
         } else {
@@ -564,7 +574,7 @@ __device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, do
           guess = true;
         }
         if (!guess) {
-          const bool still = mag_below(fabs(div_r(dtold - dtnew, dtold)), gdtol);
+          const bool still = mag_below(fabs(div_n(dtold - dtnew, dtold)), gdtol);
           if (still && mag_below(gprim, 1.0)) {
             ccount = ccount + 1;
             guess = ccount > 1;
@@ -618,7 +628,7 @@ __device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, do
         }
         counter = counter + 1;
         const double dg = gprimdernew - gprimder;
-        const double gamman = above0(dg) ? div_r(fabs((dtnew - dtold) * dg), dg * dg) : 0.0;
+        const double gamman = above0(dg) ? div_n(fabs((dtnew - dtold) * dg), dg * dg) : 0.0;
         dtold = dtnew;
         dtnew = dtnew - gamman * gprimdernew;
         bool out = false;
@@ -626,7 +636,7 @@ __device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, do
           dtnew = 0.0;
           out = true;
         } else {
-          const bool past = above1(div_r(dtnew, dt));
+          const bool past = above1(div_n(dtnew, dt));
           if (mag_below(gprim, 1.0) && past) {
             dtnew = dtold;
             guess = true;
@@ -668,11 +678,11 @@ __device__ __noinline__ double nr_time_step(double dt, double v, double dvdx, do
       phase = NEWTON;
       counter = 0;
     }
-    if (!(lt_any(nrtol, fabs(div_r(nrerror, dtnew))) && (counter < maxIter))) break;
+    if (!(lt_any(nrtol, fabs(div_n(nrerror, dtnew))) && (counter < maxIter))) break;
     at = dtnew;
   }
   if (lt_any(dt, dtnew)) return dt;
-  if ((counter == maxIter) && lt_any(nrtol, fabs(div_r(nrerror, dtnew)))) return 0.0;
+  if ((counter == maxIter) && lt_any(nrtol, fabs(div_n(nrerror, dtnew)))) return 0.0;
   return dtnew;
 }
 
@@ -883,9 +893,9 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t ma
   R ax, ay, az;
   auto advect = [&]() {
     if constexpr (EXP) {
-      ax = (R)adv_exponential((double)vx, dvx, dt, exp(dvx * dt) - 1.0);
-      ay = (R)adv_exponential((double)vy, dvy, dt, exp(dvy * dt) - 1.0);
-      az = (R)adv_exponential((double)vz, dvz, dt, exp(dvz * dt) - 1.0);
+      ax = (R)exp_displacement((double)vx, dvx, dt);
+      ay = (R)exp_displacement((double)vy, dvy, dt);
+      az = (R)exp_displacement((double)vz, dvz, dt);
     } else {
       ax = vx * rdt;
       ay = vy * rdt;
@@ -1107,8 +1117,8 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t ma
       const R vp = p0 ? vx : vy, vq = q2 ? vz : vy;
       R ap, aq;
       if constexpr (EXP) {
-        ap = (R)adv_exponential((double)vp, dvp, dt, exp(dvp * dt) - 1.0);
-        aq = (R)adv_exponential((double)vq, dvq, dt, exp(dvq * dt) - 1.0);
+        ap = (R)exp_displacement((double)vp, dvp, dt);
+        aq = (R)exp_displacement((double)vq, dvq, dt);
       } else {
         ap = vp * rdt;
         aq = vq * rdt;
