@@ -718,10 +718,11 @@ struct Visit {
   R sqrt_dtcell, rdt_cell;
   int exitFace, posRestart;
   bool reachedMax;
+  int waits;  // passes a leaving lane has waited (EXPONENTIAL)
   int64_t passes;
 };
 
-enum : int { PASS_CONTINUE = 0, PASS_MAXTIME = 1, PASS_EXIT = 2, PASS_UNDEFINED = 3 };
+enum : int { PASS_CONTINUE = 0, PASS_MAXTIME = 1, PASS_EXIT = 2, PASS_UNDEFINED = 3, PASS_WAIT = 4 };
 
 // component k (0, 1, 2) of three values, by selects (no local-memory array)
 template <typename T>
@@ -756,6 +757,7 @@ __device__ __forceinline__ bool outside3(R a, R b, R c) {
 // field k of a slot at p[k * stride + slot]; and the EXPONENTIAL kernel's
 // per-lane values of a cell visit: the velocity gradients (V2 - V1)/D and
 // e^{gradient dtcell} - 1 per axis.
+constexpr int kLeaveEighths = 5, kMaxWaits = 16;
 constexpr int kExitSlot = 7;
 constexpr int kExpFields = 6;
 
@@ -845,12 +847,15 @@ __device__ __forceinline__ void warp_exit_solves(unsigned grp, unsigned need, co
 
 // One pass of the `do while (continueTimeLoop)` body, TrackSubCell.F90:956-1368.
 // On PASS_MAXTIME / PASS_EXIT the final location is (ox,oy,oz,V.t); on
-// PASS_UNDEFINED the caller uses the last recorded point.
+// PASS_UNDEFINED the caller uses the last recorded point; PASS_WAIT: the pass
+// has not been made.
 template <typename R, bool EXP, bool AXI>
 __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t massb, double maxTime, int ndim, int d1, int d2,
                        uint64_t seed, uint64_t id, uint64_t &ctr, R &ox, R &oy, R &oz) {
   const R zero = R(0), one = R(1), half = R(0.5);
-  const unsigned grp = __activemask();  // the lanes running this pass together
+  unsigned grp = __activemask();  // the lanes running this pass together
+  const double t_in = V.t;        // (EXPONENTIAL)
+  const uint64_t ctr_in = ctr;
   const double dtRed = (double)0.1f;  // dtReductionFactor, a single-precision literal (:850)
   double dt = V.dtcell;
   R rdt = V.rdt_cell, sdt = V.sqrt_dtcell;  // FP32 copies: no conversion on the common pass
@@ -949,6 +954,33 @@ __device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t ma
     V.reachedMax = false;
   }
   R nx = x + dxrw * iX, ny = y + dyrw * iY, nz = z + dzrw * iZ;
+  // EXPONENTIAL: leaving lanes wait until they are five of eight.  A Newton
+  // solve takes some ten passes' time and a warp runs it with the lanes that
+  // have one, so a lane that would leave stays where it was before the pass
+  // and repeats it -- the same draws, the same step; the other lanes' passes
+  // pay for it -- until enough lanes of the warp, or all, would leave, or
+  // one has waited for 16 passes (particles that seldom leave).  40,001
+  // particles of a 61x37x7 field, two 5-day intervals: 43.3 -> 34.6 ms (three of
+  // eight 38.6, four 36.5, six 35.9); 200,001, one interval: 64 -> 54.  In the
+  // EULERIAN kernels, whose solves are short, the waiting costs what it gives
+  // (FP64 50.6 -> 51.4 ms at two of eight, MIXED 10.7 -> 11.7).
+  if constexpr (EXP) {
+    __syncwarp(grp);
+    const bool leaves = MPRW_OUTSIDE(nx, ny, nz);
+    const unsigned lm = __ballot_sync(grp, leaves);
+    if (lm != grp && 8 * __popc(lm) < kLeaveEighths * __popc(grp) &&
+        !__any_sync(grp, leaves && V.waits >= kMaxWaits)) {
+      if (leaves) {
+        ++V.waits;
+        V.t = t_in;
+        V.reachedMax = false;
+        ctr = ctr_in;
+        return PASS_WAIT;
+      }
+      grp &= ~lm;
+    }
+    V.waits = 0;
+  }
   // FP64 and EXPONENTIAL: the first interface iteration's exit-face solves of
   // the leaving lanes, spread over every lane of the pass
   unsigned pre_r = 0u;
@@ -1275,6 +1307,7 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
   V.exitFace = V.posRestart = 0;
   V.reachedMax = false;
   V.passes = 0;
+  V.waits = 0;
   uint32_t massb = 0;
   // cell exits of the current particle in this launch (bits 0-19) and how
   // many of the last ones took no time (bits 20-30): one register for both caps
@@ -1409,7 +1442,8 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
         r = PASS_UNDEFINED;
       } else {
         r = rw_pass<R, EXP, AXI>(V, F, slots, massb, a.t_end, a.ndim, a.d1, a.d2, a.seed, id, ctr, ox, oy, oz);
-        ++my_passes;
+        if (EXP && r == PASS_WAIT) --V.passes;
+        else ++my_passes;
       }
       if (r == PASS_MAXTIME) {
         a.cell[p] = c; a.x[p] = ox; a.y[p] = oy; a.z[p] = oz; a.t[p] = V.t;
