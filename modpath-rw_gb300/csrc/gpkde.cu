@@ -462,8 +462,10 @@ __global__ void __launch_bounds__(kThreads) key_assign_kernel(KdeParams P, KdeBi
       int key = -1;
       if (in) {
         const T s = B.support[b];
+        // (cells of equal sides: one level for all)
         for (int d = 0; d < 3; ++d)
-          if (P.mask[d]) lev[d] = log_index<T>(P, s, d);
+          if (P.mask[d])
+            lev[d] = d > 0 && P.mask[d - 1] && P.bin[d] == P.bin[d - 1] ? lev[d - 1] : log_index<T>(P, s, d);
         key = lev[0] + lev[1] + lev[2] - 3;
         bin_key[b] = key;
       }
@@ -538,15 +540,20 @@ static_assert(kThreads == kPlanThreads, "the key assignment's last block runs th
 __device__ void plan_body(const KdeParams &P, KeyAcc *K, const KdeTable &t0, const KdeTable &t1,
                           const KdeTable &t2, int scatter, SepPlan *pl, int nc, long long cap1, long long cap2,
                           long long *need, double *S, int work_weight) {
-  __shared__ long long sv1[kPlanThreads], sv2[kPlanThreads];
-  __shared__ int sp[kPlanThreads];
+  __shared__ long long wv1[kPlanThreads / 32], wv2[kPlanThreads / 32];
+  __shared__ int wp[kPlanThreads / 32];
   __shared__ int su[3][6];
   const int k = threadIdx.x;
   if (k < 3) {
     su[k][0] = su[k][2] = su[k][4] = INT_MAX;
     su[k][1] = su[k][3] = su[k][5] = INT_MIN;
   }
-  const int cntk = k < KDE_KMAX ? __ldcg(&K->cnt[k]) : 0;
+  // (all loads in flight together: the plan is a chain of them)
+  const int kk = min(k, KDE_KMAX - 1);
+  int lv[3], kb[6];
+  for (int d = 0; d < 3; ++d) lv[d] = __ldcg(&K->lev[kk][d]);
+  for (int i = 0; i < 6; ++i) kb[i] = __ldcg(&K->box[kk][i]);
+  const int cntk = k < KDE_KMAX ? __ldcg(&K->cnt[kk]) : 0;
   const bool present = cntk > 0;
   int m[3] = {0, 0, 0}, fo[3] = {0, 0, 0}, bx[6], r1[6], r2[6];
   long long v1 = 0, v2 = 0;
@@ -554,11 +561,11 @@ __device__ void plan_body(const KdeParams &P, KeyAcc *K, const KdeTable &t0, con
     const int axis = k / KDE_MAXDB;
     const KdeTable T = !scatter ? t0 : (axis == 0 ? t0 : (axis == 1 ? t1 : t2));
     for (int d = 0; d < 3; ++d) {
-      const int li = d * KDE_MAXDB + __ldcg(&K->lev[k][d]) - 1;
+      const int li = d * KDE_MAXDB + lv[d] - 1;
       m[d] = T.m[li];
       fo[d] = T.ofs[li];
     }
-    for (int i = 0; i < 6; ++i) bx[i] = r1[i] = r2[i] = __ldcg(&K->box[k][i]);
+    for (int i = 0; i < 6; ++i) bx[i] = r1[i] = r2[i] = kb[i];
     if (!scatter) {
       r1[2] = max(1, bx[2] - m[1]);
       r1[3] = min(P.nb[1], bx[3] + m[1]);
@@ -577,23 +584,40 @@ __device__ void plan_body(const KdeParams &P, KeyAcc *K, const KdeTable &t0, con
       atomicAdd(work_counter(S), (unsigned long long)cntk * (unsigned long long)work_weight *
                                      (unsigned long long)((2 * m[0] + 1) * (2 * m[1] + 1) * (2 * m[2] + 1)));
   }
-  sp[k] = present ? 1 : 0;
-  sv1[k] = v1;
-  sv2[k] = v2;
-  __syncthreads();
-  // inclusive Hillis-Steele scans
-  for (int o = 1; o < kPlanThreads; o <<= 1) {
-    const int a = (k >= o) ? sp[k - o] : 0;
-    const long long b1 = (k >= o) ? sv1[k - o] : 0, b2 = (k >= o) ? sv2[k - o] : 0;
-    __syncthreads();
-    sp[k] += a;
-    sv1[k] += b1;
-    sv2[k] += b2;
-    __syncthreads();
+  // inclusive scans: within the warps, then over the warps' totals
+  const int lane = k & 31, w = k >> 5;
+  int p = present ? 1 : 0;
+  long long s1 = v1, s2 = v2;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, p, o);
+    const long long b1 = __shfl_up_sync(0xffffffffu, s1, o), b2 = __shfl_up_sync(0xffffffffu, s2, o);
+    if (lane >= o) {
+      p += a;
+      s1 += b1;
+      s2 += b2;
+    }
   }
-  if (k < KDE_KMAX) pl->slot_of[k] = present ? sp[k] - 1 : -1;
+  if (lane == 31) {
+    wp[w] = p;
+    wv1[w] = s1;
+    wv2[w] = s2;
+  }
+  __syncthreads();
+  int np = 0;
+  long long tot1 = 0, tot2 = 0;
+  for (int i = 0; i < kPlanThreads / 32; ++i) {
+    if (i < w) {
+      p += wp[i];
+      s1 += wv1[i];
+      s2 += wv2[i];
+    }
+    np += wp[i];
+    tot1 += wv1[i];
+    tot2 += wv2[i];
+  }
+  if (k < KDE_KMAX) pl->slot_of[k] = present ? p - 1 : -1;
   if (present) {
-    const int j = sp[k] - 1;
+    const int j = p - 1;
     for (int d = 0; d < 3; ++d) {
       pl->m[j][d] = m[d];
       pl->fofs[j][d] = fo[d];
@@ -603,8 +627,8 @@ __device__ void plan_body(const KdeParams &P, KeyAcc *K, const KdeTable &t0, con
       pl->r1[j][i] = r1[i];
       pl->r2[j][i] = r2[i];
     }
-    pl->o1[j] = sv1[k] - v1;
-    pl->o2[j] = sv2[k] - v2;
+    pl->o1[j] = s1 - v1;
+    pl->o2[j] = s2 - v2;
     pl->key[j] = k;
     if (scatter) {
       const int axis = k / KDE_MAXDB;
@@ -623,9 +647,6 @@ __device__ void plan_body(const KdeParams &P, KeyAcc *K, const KdeTable &t0, con
     K->box[k][1] = K->box[k][3] = K->box[k][5] = INT_MIN;
     K->cnt[k] = 0;
   }
-  // totals: the inclusive scans end at the last key
-  const int np = sp[kPlanThreads - 1];
-  const long long tot1 = sv1[kPlanThreads - 1], tot2 = sv2[kPlanThreads - 1];
   __syncthreads();  // su complete
   const bool fits = tot1 * nc <= cap1 && tot2 * nc <= cap2;
   if (k < 3)
@@ -1355,10 +1376,14 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // npts2: nPoints**fTWO, which Fortran evaluates as the product nPoints*nPoints
 
+// The last block to finish folds the partials -- warp 0's lane l partials l,
+// l + 32, ..., then a shuffle tree -- which as a kernel of its own took 3 us
+// and its place in the graph.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) bin_reduce_kernel(KdeParams P, KdeBinsT<T> B, int what, double npts2,
-                                                              const double *S, double *partial) {
+                                                              double *S, double *partial, unsigned int *done) {
   __shared__ double red[kThreads / 32][3];
+  __shared__ bool last;
   double a[3] = {0.0, 0.0, 0.0};
   const double mx = S[S_DMAX], mx_old = S[S_DMAXOLD];
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B.n; b += gridDim.x * blockDim.x) {
@@ -1393,17 +1418,19 @@ __global__ void __launch_bounds__(kThreads) bin_reduce_kernel(KdeParams P, KdeBi
       for (int i = 1; i < kThreads / 32; ++i) v = v + red[i][k];
       partial[3 * blockIdx.x + k] = v;
     }
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
   }
-}
-
-// one warp: lane l folds partials l, l+32, ... then a shuffle tree
-__global__ void bin_reduce_final_kernel(int what, int nblk, const double *partial, double *S) {
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  __threadfence();
   const int l = threadIdx.x;
-  double a[3] = {0.0, 0.0, 0.0};
-  for (int i = l; i < nblk; i += 32)
-    for (int k = 0; k < 3; ++k) a[k] = a[k] + partial[3 * i + k];
+  a[0] = a[1] = a[2] = 0.0;
+  for (int i = l; i < gridDim.x; i += 32)
+    for (int k = 0; k < 3; ++k) a[k] = a[k] + __ldcg(&partial[3 * i + k]);
   for (int k = 0; k < 3; ++k) a[k] = warp_sum(a[k]);
   if (l != 0) return;
+  *done = 0u;  // for the next reduction (kernel boundaries order it)
   if (what == RED_END) {
     S[S_ERRD] = a[0];
     S[S_ERRS] = a[1];
@@ -1648,7 +1675,9 @@ cudaError_t KdeState::ensure_grid(int64_t ngrid) {
     cudaError_t e = cudaMalloc((void **)&d_scalars, 32 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_wcnt, 64 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMallocHost((void **)&h_scalars, 96 * sizeof(double));  // + the 64 counters
-    if (e == cudaSuccess) e = cudaMalloc((void **)&d_flag, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&d_flag, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(d_flag, 0, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // (the handle's stream does not wait for it)
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_keys, sizeof(KeyAcc));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_plan, 2 * sizeof(SepPlan));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_need, 4 * sizeof(long long));
@@ -2043,9 +2072,9 @@ static cudaError_t kde_attempt(KdeState &st, const KdeParams &P, double hs, doub
     return cudaGetLastError();
   };
   auto reduce = [&](int what) -> cudaError_t {
-    bin_reduce_kernel<T><<<rb, kThreads, 0, s>>>(P, B, what, npts * npts, S, st.partial);
-    bin_reduce_final_kernel<<<1, 32, 0, s>>>(what, rb, st.partial, S);
-    st.launches += 2;
+    bin_reduce_kernel<T><<<rb, kThreads, 0, s>>>(P, B, what, npts * npts, S, st.partial,
+                                                 reinterpret_cast<unsigned int *>(st.d_flag + 1));
+    st.launches += 1;
     return cudaGetLastError();
   };
   auto fetch_async = [&](void) -> cudaError_t {

@@ -96,7 +96,8 @@ struct KdeState {
   double *dens_out = nullptr;                             // FP64 output grid
   int64_t grid_cap = 0;
   double *partial = nullptr, *d_scalars = nullptr, *h_scalars = nullptr;
-  int *d_flag = nullptr, *d_blockcnt = nullptr;
+  int *d_flag = nullptr;  // optimal smoothing clipped somewhere; the reductions' finished blocks
+  int *d_blockcnt = nullptr;
   int *cell_bin = nullptr;          // per grid cell: active bin index or -1
   int *bin_key = nullptr;           // per bin: smoothing key (n) and SD keys per axis (3n)
   KeyAcc *d_keys = nullptr;
