@@ -215,6 +215,18 @@ constexpr int kWarpsW = 4;
 constexpr int kRowCache = 256;
 static_assert(kRowCache >= KDE_MAXLEN, "one layer of a span's rows fits the row cache");
 
+// v >= 0 (below 2^62) rounded to an integer, to even at a half: from 2^23 on
+// the significand shifted; below, 2^23 + v rounds to the integer above the
+// pattern of 2^23.  The conversion to 64 bits is one of GB300's slow ones: nine
+// scatters of 300,000 particles on 187 x 93 x 21 bins 0.52 -> 0.46 ms.
+__device__ __forceinline__ unsigned long long fixed_rn(float v) {
+  const unsigned u = __float_as_uint(v);
+  const int e = (int)(u >> 23);
+  const unsigned lo = __float_as_uint(v + 8388608.0f) - 0x4B000000u;
+  const unsigned long long hi = (unsigned long long)((u & 0x7FFFFFu) | 0x800000u) << ((e - 150) & 63);
+  return e < 150 ? (unsigned long long)lo : hi;
+}
+
 // round(a * b / 2^63) for a < 2^63, b <= 2^63 (the 128-bit product, rounded
 // to nearest), on the integer pipe
 __device__ __forceinline__ unsigned long long mulq63(unsigned long long a, unsigned long long b) {
@@ -290,9 +302,10 @@ __global__ void __launch_bounds__(32 * kWarpsW) wscatter_kernel(KdeParams P, Kde
   // constant from layer to layer -- so the inner loop is a load, the cell's
   // product and the addition, on full warps whatever the span's width.  (Lanes
   // along x only: a span of 21 cells left 11 of 32 idle, and every cell
-  // worked out its row's indexes.)  What bounds it: FP32 the conversions to
-  // 64-bit integers (without the additions it takes as long), FP64 the integer
-  // products.  1,000,000 particles on 200 x 100 x 20 bins, nine scatters:
+  // worked out its row's indexes.)  What bounds it: the integer work per cell
+  // (FP64 products, FP32 conversions; without the additions the widest kernels
+  // take four fifths of the time), for small kernels the loads before it.
+  // 1,000,000 particles on 200 x 100 x 20 bins, nine scatters:
   // FP64 1.04 -> 0.64 ms (0.18 of it from sizing the factors' shared memory by
   // the database instead of its largest legal one, which doubles the resident
   // warps); 300,000 on 187 x 93 x 21, FP32: 0.59 -> 0.52 ms.
@@ -342,8 +355,10 @@ __global__ void __launch_bounds__(32 * kWarpsW) wscatter_kernel(KdeParams P, Kde
   } else {
     // (the scale is a power of two: applied to the row product it gives the
     // same rounded cell products)
-    spread([&](int iy, int iz) { return cnt * (fy[iy] * fz[iz]) * fscale; }, fx,
-           [&](T r, T f) { return (unsigned long long)__float2ll_rn(r * f); }, crow_all[w]);
+    const T cm = fabsf(cnt);
+    const unsigned long long sgn = cnt < T(0) ? ~0ull : 0ull;
+    spread([&](int iy, int iz) { return cm * (fy[iy] * fz[iz]) * fscale; }, fx,
+           [&](T r, T f) { return (fixed_rn(r * f) ^ sgn) - sgn; }, crow_all[w]);
   }
 }
 

@@ -92,3 +92,25 @@ def test_small_reconstruction_on_a_stream_and_on_the_default_stream(gpu_lib):
         np.testing.assert_array_equal(h0, h1)
         assert np.array_equal(d0.view(np.uint64), d1.view(np.uint64))
     tr.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3])
+def test_few_particles_in_fp32(gpu_lib, n):
+    """The FP32 scatter's fixed-point cell products at their largest scale:
+    one particle's kernel spans from its centre to its last cell every
+    magnitude from 2^60 units down, some below 2^23 (rounded) and most above
+    (shifted).  Against FP64 to 1e-3 of the maximum and the mass to 1e-4, as
+    test_gpu_gpkde."""
+    g, f, p, opt, _ = W.lognormal_slab(n_particles=8, nlay=9, nrow=21, ncol=21, seed=7, use_torch=False)
+    p = W.release_in_box(g, n, 9.0, 12.0, 9.0, 12.0, float(g.botm[-1]), float(g.top[0]), seed=8)
+    tr = mprw.Tracker(g, opt)
+    tr.load_flow(f)
+    tr.set_particles(p)
+    tr.advance(0.0, 0.001)
+    d64, h64, l64 = tr.gpkde((21.0, 21.0, 9.0), (1.0, 1.0, 1.0), n_opt_loops=0)
+    d32, h32, l32 = tr.gpkde((21.0, 21.0, 9.0), (1.0, 1.0, 1.0), n_opt_loops=0, precision=MIXED)
+    tr.close()
+    np.testing.assert_array_equal(h32, h64)
+    assert h64.sum() == n and d64.max() > 0
+    np.testing.assert_allclose(d32, d64, rtol=0, atol=1e-3 * d64.max())
+    assert abs(d32.sum() - d64.sum()) < 1e-4 * n
