@@ -796,7 +796,7 @@ int max_blocks_per_sm(mprw_handle *h) {
 }
 
 // EXPONENTIAL: particles from which every resident warp is filled
-constexpr int64_t kExpSpread = 150000;
+constexpr int64_t kExpSpread = 80000;
 
 int default_blocks_per_sm(mprw_handle *h) {
   // EULERIAN MIXED is compiled for 3 resident blocks per SM (80 registers)
@@ -819,8 +819,9 @@ struct StepShape {
 // latency), then few lanes per warp, two at least.  Measured, two intervals
 // (ms, all warps full -> spread): FP64 column of 2,000 particles 2.39 -> 1.15,
 // 30,000: 2.55 -> 1.80; FP64 100x60x10 field, 4,000: 8.35 -> 5.77, 16,000: 9.29
-// -> 7.0; MIXED, 4,000: 3.23 -> 1.97; EXPONENTIAL, 4,000: 39 -> 18, 40,000: 52 ->
-// 41 (150,000: equal).  Past one particle per lane the FP64 warps are levelled
+// -> 7.0; MIXED, 4,000: 3.23 -> 1.97; EXPONENTIAL, 61x37x7 field, 4,000: 13.3 ->
+// 8.2 (one interval), 40,000: 37.4 -> 30.4, 80,000: 24.1 and 24.7 (one interval),
+// 150,000: 36.8 filled, 41.2 spread.  Past one particle per lane the FP64 warps are levelled
 // over the rounds (100,000 particles, 12 warps -> 11: 7.07 -> 6.71); MIXED runs
 // blocks of four warps (1,000,000: equal; 40,000 in the column: 0.78 -> 0.70).
 StepShape step_shape(mprw_handle *h, int bps) {
