@@ -1087,12 +1087,31 @@ __global__ void gather_z_kernel(KdeParams P, KdeBinsT<T> B, const SepPlan *pl, c
     const int bx = B.gx[b], by = B.gy[b], bz = B.gz[b];
     const int *r2 = pl->r2[j];
     const T *in = T2 + pl->o2[j] * NC;
-    for (int t = sub; t <= 2 * m; t += LPB) {
-      const int p = reflect_pos(bz - m + t, n);
-      if (p < 1) continue;
+    // (positions that fold to nowhere lie at the window's ends; four taps'
+    // loads, or two of several fields, in flight before their sums, which stay
+    // in the taps' order: with one tap's at a time a launch of 56,000 bins took
+    // 25.1 us for 19.3, in FP32 8.6 for 7.1 at 43,000)
+    constexpr int U = NC == 1 ? 4 : 2;
+    const long long st = (long long)(r2[1] - r2[0] + 1) * (r2[3] - r2[2] + 1) * NC;
+    const T *col = in + (region_loc(r2, bx, by, r2[4]) * NC - r2[4] * st);
+    const int lo = max(0, 1 - 2 * n - (bz - m)), t1 = min(2 * m, 2 * n - (bz - m));
+    int t = lo + (sub - lo % LPB + LPB) % LPB;
+    for (; t + (U - 1) * LPB <= t1; t += U * LPB) {
+      T w[U], v[U][NC];
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        w[k] = f[t + k * LPB];
+        const T *q = col + reflect_pos(bz - m + t + k * LPB, n) * st;
+        for (int c = 0; c < NC; ++c) v[k][c] = q[c];
+      }
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        for (int c = 0; c < NC; ++c) acc[c] += w[k] * v[k][c];
+    }
+    for (; t <= t1; t += LPB) {
       const T w = f[t];
-      const long long l = region_loc(r2, bx, by, p) * NC;
-      for (int c = 0; c < NC; ++c) acc[c] += w * in[l + c];
+      const T *q = col + reflect_pos(bz - m + t, n) * st;
+      for (int c = 0; c < NC; ++c) acc[c] += w * q[c];
     }
   }
   if constexpr (LPB > 1) {
