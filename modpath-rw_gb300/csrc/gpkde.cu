@@ -758,58 +758,41 @@ __device__ __forceinline__ void gx_element(const KdeParams &P, const SepPlan *pl
   const long long row = (long long)P.nb[0] * ((y - 1) + (long long)P.nb[1] * (z - 1)) - 1;
   T acc[NC];
   for (int c = 0; c < NC; ++c) acc[c] = T(0);
-  if constexpr (sizeof(T) == 8) {
-    // One loop for windows inside and across the edges.  The FP64 pipe holds a
-    // warp's multiply-add for 16 clocks whatever its lanes, and a warp mostly
-    // has both kinds of window; as two loops (the FP32 form below) its
-    // multiply-adds ran on 16 of 32 lanes.  The fold is integer work beside
-    // them, and positions that fold to nowhere lie at the ends of the window.
-    // 1,000,000 particles on 200 x 100 x 20 bins: the 24 x passes of a
-    // reconstruction 2.26 -> 1.56 ms, the y passes 1.31 -> 1.19 ms.
-    T acc2[NC];
-    for (int c = 0; c < NC; ++c) acc2[c] = T(0);
-    const int t1 = min(2 * m, 2 * n - x + m);
-    int t = max(0, 1 - 2 * n - x + m);
-    for (; t < t1; t += 2) {
-      const T w0 = f[t], w1 = f[t + 1];
-      const long long l0 = row + reflect_pos(x - m + t, n), l1 = row + reflect_pos(x - m + t + 1, n);
-      for (int c = 0; c < NC; ++c) {
-        acc[c] += w0 * F.f[c][l0];
-        acc2[c] += w1 * F.f[c][l1];
-      }
+  // One loop for windows inside and across the edges, which a warp mostly has
+  // both of (positions that fold to nowhere lie at the window's ends).  As two
+  // loops FP64's multiply-adds, 16 clocks of the pipe each whatever the lanes,
+  // ran on 16 of 32 of them: 1,000,000 particles on 200 x 100 x 20 bins, the 24
+  // x passes of a reconstruction 2.26 -> 1.56 ms, the y passes 1.31 -> 1.19; in
+  // FP32 one loop's latency followed the other's: 300,000 on 187 x 93 x 21, 0.44
+  // -> 0.36 and 0.51 -> 0.46 ms.  Two partial sums run ahead of each other, but
+  // for FP32's windows across an edge, which have one.
+  auto at = [&](int c, int p) { return F.f[c][row + p]; };
+  T acc2[NC];
+  for (int c = 0; c < NC; ++c) acc2[c] = T(0);
+  const bool two = sizeof(T) == 8 || (x - m >= 1 && x + m <= n);
+  const int t1 = min(2 * m, 2 * n - x + m);
+  int t = max(0, 1 - 2 * n - x + m);
+  for (; t < t1; t += 2) {
+    const T w0 = f[t], w1 = f[t + 1];
+    const int p0 = reflect_pos(x - m + t, n), p1 = reflect_pos(x - m + t + 1, n);
+    T v0[NC], v1[NC];
+    for (int c = 0; c < NC; ++c) {
+      v0[c] = at(c, p0);
+      v1[c] = at(c, p1);
     }
-    if (t == t1) {
-      const T w0 = f[t];
-      const long long l0 = row + reflect_pos(x - m + t, n);
-      for (int c = 0; c < NC; ++c) acc[c] += w0 * F.f[c][l0];
-    }
-    for (int c = 0; c < NC; ++c) acc[c] += acc2[c];
-  } else if (x - m >= 1 && x + m <= n) {
-    // the window misses both edges: a straight loop, two partial sums per
-    // field so that the loads run ahead of the multiply-adds
-    T acc2[NC];
-    for (int c = 0; c < NC; ++c) acc2[c] = T(0);
-    const long long base = row + x - m;
-    int t = 0;
-#pragma unroll 2
-    for (; t + 1 <= 2 * m; t += 2) {
-      const T w0 = f[t], w1 = f[t + 1];
-      for (int c = 0; c < NC; ++c) {
-        acc[c] += w0 * F.f[c][base + t];
-        acc2[c] += w1 * F.f[c][base + t + 1];
-      }
-    }
-    if (t <= 2 * m)
-      for (int c = 0; c < NC; ++c) acc[c] += f[t] * F.f[c][base + t];
-    for (int c = 0; c < NC; ++c) acc[c] += acc2[c];
-  } else {
-    for (int t = 0; t <= 2 * m; ++t) {
-      const int p = reflect_pos(x - m + t, n);
-      if (p < 1) continue;
-      const T w = f[t];
-      for (int c = 0; c < NC; ++c) acc[c] += w * F.f[c][row + p];
+    for (int c = 0; c < NC; ++c) {
+      acc[c] += w0 * v0[c];
+      if (two) acc2[c] += w1 * v1[c];
+      else acc[c] += w1 * v1[c];
     }
   }
+  if (t == t1) {
+    const T w0 = f[t];
+    const int p0 = reflect_pos(x - m + t, n);
+    for (int c = 0; c < NC; ++c) acc[c] += w0 * at(c, p0);
+  }
+  if (two)
+    for (int c = 0; c < NC; ++c) acc[c] += acc2[c];
   for (int c = 0; c < NC; ++c) out[i * NC + c] = acc[c];
 }
 
@@ -983,55 +966,36 @@ __device__ __forceinline__ void gy_element(const KdeParams &P, const SepPlan *pl
   region_xyz(r2, i, x, y, z);
   T acc[NC];
   for (int c = 0; c < NC; ++c) acc[c] = T(0);
-  if constexpr (sizeof(T) == 8) {
-    T acc2[NC];
-    for (int c = 0; c < NC; ++c) acc2[c] = T(0);
-    const int st = (r1[1] - r1[0] + 1) * NC;
-    const T *src = in + region_loc(r1, x, r1[2], z) * NC - (long long)r1[2] * st;
-    const int t1 = min(2 * m, 2 * n - y + m);
-    int t = max(0, 1 - 2 * n - y + m);
-    for (; t < t1; t += 2) {
-      const T w0 = f[t], w1 = f[t + 1];
-      const T *s0 = src + (long long)reflect_pos(y - m + t, n) * st;
-      const T *s1 = src + (long long)reflect_pos(y - m + t + 1, n) * st;
-      for (int c = 0; c < NC; ++c) {
-        acc[c] += w0 * s0[c];
-        acc2[c] += w1 * s1[c];
-      }
+  // one loop, as in the x pass
+  const long long st = (long long)(r1[1] - r1[0] + 1) * NC;
+  const T *src = in + region_loc(r1, x, r1[2], z) * NC - r1[2] * st;
+  auto at = [&](int c, int p) { return src[p * st + c]; };
+  T acc2[NC];
+  for (int c = 0; c < NC; ++c) acc2[c] = T(0);
+  const bool two = sizeof(T) == 8 || (y - m >= 1 && y + m <= n);
+  const int t1 = min(2 * m, 2 * n - y + m);
+  int t = max(0, 1 - 2 * n - y + m);
+  for (; t < t1; t += 2) {
+    const T w0 = f[t], w1 = f[t + 1];
+    const int p0 = reflect_pos(y - m + t, n), p1 = reflect_pos(y - m + t + 1, n);
+    T v0[NC], v1[NC];
+    for (int c = 0; c < NC; ++c) {
+      v0[c] = at(c, p0);
+      v1[c] = at(c, p1);
     }
-    if (t == t1) {
-      const T w0 = f[t];
-      const T *s0 = src + (long long)reflect_pos(y - m + t, n) * st;
-      for (int c = 0; c < NC; ++c) acc[c] += w0 * s0[c];
-    }
-    for (int c = 0; c < NC; ++c) acc[c] += acc2[c];
-  } else if (y - m >= 1 && y + m <= n) {
-    // interior window (inside region 1 by construction): straight loop
-    T acc2[NC];
-    for (int c = 0; c < NC; ++c) acc2[c] = T(0);
-    const T *src = in + region_loc(r1, x, y - m, z) * NC;
-    const long long st = (long long)(r1[1] - r1[0] + 1) * NC;
-    int t = 0;
-#pragma unroll 2
-    for (; t + 1 <= 2 * m; t += 2) {
-      const T w0 = f[t], w1 = f[t + 1];
-      for (int c = 0; c < NC; ++c) {
-        acc[c] += w0 * src[t * st + c];
-        acc2[c] += w1 * src[(t + 1) * st + c];
-      }
-    }
-    if (t <= 2 * m)
-      for (int c = 0; c < NC; ++c) acc[c] += f[t] * src[t * st + c];
-    for (int c = 0; c < NC; ++c) acc[c] += acc2[c];
-  } else {
-    for (int t = 0; t <= 2 * m; ++t) {
-      const int p = reflect_pos(y - m + t, n);
-      if (p < 1) continue;
-      const T w = f[t];
-      const long long l = region_loc(r1, x, p, z) * NC;
-      for (int c = 0; c < NC; ++c) acc[c] += w * in[l + c];
+    for (int c = 0; c < NC; ++c) {
+      acc[c] += w0 * v0[c];
+      if (two) acc2[c] += w1 * v1[c];
+      else acc[c] += w1 * v1[c];
     }
   }
+  if (t == t1) {
+    const T w0 = f[t];
+    const int p0 = reflect_pos(y - m + t, n);
+    for (int c = 0; c < NC; ++c) acc[c] += w0 * at(c, p0);
+  }
+  if (two)
+    for (int c = 0; c < NC; ++c) acc[c] += acc2[c];
   for (int c = 0; c < NC; ++c) out[i * NC + c] = acc[c];
 }
 
