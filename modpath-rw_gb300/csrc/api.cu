@@ -821,7 +821,8 @@ struct StepShape {
 // 30,000: 2.55 -> 1.80; FP64 100x60x10 field, 4,000: 8.35 -> 5.77, 16,000: 9.29
 // -> 7.0; MIXED, 4,000: 3.23 -> 1.97; EXPONENTIAL, 61x37x7 field, 4,000: 13.3 ->
 // 8.2 (one interval), 40,000: 37.4 -> 30.4, 80,000: 24.1 and 24.7 (one interval),
-// 150,000: 36.8 filled, 41.2 spread.  Past one particle per lane the FP64 warps are levelled
+// 150,000: 36.8 filled, 41.2 spread (first intervals in cell order; 21.8 and 34.2
+// heaviest first).  Past one particle per lane the FP64 warps are levelled
 // over the rounds (100,000 particles, 12 warps -> 11: 7.07 -> 6.71); MIXED runs
 // blocks of four warps (1,000,000: equal; 40,000 in the column: 0.78 -> 0.70).
 StepShape step_shape(mprw_handle *h, int bps) {
@@ -954,7 +955,26 @@ int launch_step(mprw_handle *h, double t_begin, double t_end, int bps, bool use_
 
 int sort_particles(mprw_handle *h) {
   const uint64_t per_pass = 3ull * (uint64_t)h->ndim;  // Philox blocks per pass: 3 per normal, ndim normals
-  CK(sort_cells(h->d_cell, h->d_ctr, h->ctr_prev_valid ? h->d_ctr_prev : nullptr, per_pass, h->d_perm, h->n,
+  PassGuess g{};
+  if (h->opt.precision == MPRW_MIXED) {
+    g.dtcell = reinterpret_cast<const char *>(&h->d_rec32->dtcell);
+    g.stride = sizeof(CellRec<float>);
+  } else {
+    g.dtcell = reinterpret_cast<const char *>(&h->d_rec64->dtcell);
+    g.stride = sizeof(CellRec<double>);
+  }
+  g.t = h->d_t;
+  g.t_begin = h->last_t_begin;
+  g.t_end = h->last_t_end;
+  // Heaviest first pays where warps take more than one round of particles; in
+  // one round it only puts the long ones onto the same SMs (50,000 particles,
+  // FP64, three intervals of five days: 1.9 1.7 1.6 ms by cell, 2.5 1.9 1.9
+  // heaviest first).  EXPONENTIAL, whose long particles' solves slow each other
+  // down, from two rounds on (10,000, 1.6 rounds: 11.3 against 12.2 ms).
+  const StepShape shape = step_shape(h, h->blocks_per_sm > 0 ? h->blocks_per_sm : default_blocks_per_sm(h));
+  const int64_t lanes = shape.blocks * (shape.threads / 32) * shape.lanes;
+  const bool by_cell = h->n <= (h->opt.advection_kind == 1 ? 2 * lanes : lanes);
+  CK(sort_cells(h->d_cell, by_cell ? nullptr : h->d_ctr, h->ctr_prev_valid ? h->d_ctr_prev : nullptr, per_pass, g, h->d_perm, h->n,
                 h->ncell_bits, &h->scratch, &h->scratch_bytes, h->stream));
   h->launches += 2;
   h->perm_valid = true;

@@ -47,3 +47,33 @@ def test_results_do_not_depend_on_the_launch_shape(gpu_lib, precision, advection
         for k in KEYS:
             np.testing.assert_array_equal(o[k], full[k][a:b], err_msg=f"{a}:{b} {k}")
     assert total == steps
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+def test_results_do_not_depend_on_the_processing_order(gpu_lib, precision):
+    """Particles are taken heaviest first: by their passes of the previous
+    advance, or by the time they have over their cell's time step.  With that
+    order and with none: active and pending particles, a second interval, the
+    same particles handed over again, a different number of them."""
+    n = 130_000   # more than one round of lanes in either precision
+    g, f, p, opt, _ = W.lognormal_slab(n_particles=n, nlay=4, nrow=12, ncol=30, seed=13, precision=precision,
+                                       use_torch=False)
+    rng = np.random.default_rng(3)
+    p.status = np.where(rng.random(n) < 0.3, 0, p.status).astype(p.status.dtype)
+    p.t = np.where(p.status == 0, rng.uniform(0.0, 7.0, n), 0.0)
+    out = []
+    for interval in (1, 0):
+        tr = mprw.Tracker(g, opt)
+        tr.load_flow(f)
+        tr.set_tuning(0, interval)
+        states = []
+        for sel in (slice(0, n), slice(0, n), slice(0, 500)):
+            tr.set_particles(_part(p, sel))
+            for a, b in ((0.0, 4.0), (4.0, 6.0)):
+                states.append((tr.advance(a, b), tr.get_particles(global_xyz=False)))
+        tr.close()
+        out.append(states)
+    for (s0, a), (s1, b) in zip(*out):
+        assert s0 == s1 > 0
+        for k in KEYS:
+            np.testing.assert_array_equal(a[k], b[k], err_msg=k)
