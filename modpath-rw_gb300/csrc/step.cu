@@ -817,7 +817,7 @@ constexpr int kExpFields = 6;
 // once (bit k of rbits), its exit face and its time.  Without this, a warp
 // solves its lanes' first leaving axes together and then their second axes
 // (corner crossings) in a second round of one or two lanes.  Every lane of
-// grp calls it together.  The operands travel through the warp's exchange
+// grp calls it together, and no other lane of the warp.  The operands travel through the warp's exchange
 // slots in shared memory: the owner of task t writes slot t, the lane of that
 // rank reads it and writes the result back, so nobody searches for an owner.
 template <typename R, bool EXP>
@@ -894,12 +894,12 @@ __device__ __forceinline__ void warp_exit_solves(unsigned grp, unsigned need, co
 // One pass of the `do while (continueTimeLoop)` body, TrackSubCell.F90:956-1368.
 // On PASS_MAXTIME / PASS_EXIT the final location is (ox,oy,oz,V.t); on
 // PASS_UNDEFINED the caller uses the last recorded point; PASS_WAIT: the pass
-// has not been made.
+// has not been made.  `grp` (FP64, EXPONENTIAL): the lanes of the warp that
+// call this together.
 template <typename R, bool EXP, bool AXI>
-__device__ int rw_pass(Visit<R> &V, const Lane<R> &F, double *slots, uint32_t massb, double maxTime, int ndim, int d1, int d2,
+__device__ int rw_pass(unsigned grp, Visit<R> &V, const Lane<R> &F, double *slots, uint32_t massb, double maxTime, int ndim, int d1, int d2,
                        uint64_t seed, uint64_t id, uint64_t &ctr, R &ox, R &oy, R &oz) {
   const R zero = R(0), one = R(1), half = R(0.5);
-  unsigned grp = __activemask();  // the lanes running this pass together
   const double t_in = V.t;        // (EXPONENTIAL)
   const uint64_t ctr_in = ctr;
   const double dtRed = (double)0.1f;  // dtReductionFactor, a single-precision literal (:850)
@@ -1480,14 +1480,21 @@ __global__ void __launch_bounds__(step_threads(sizeof(R) == 8, EXP), (sizeof(R) 
       }
     }
 
-    // (c) one time-loop pass (with the per-visit safety cap)
-    if (p >= 0 && !need_cell) {
+    // (c) one time-loop pass (with the per-visit safety cap).  Its lanes are
+    // settled by a vote of the whole warp: cell entry has just divided it, and
+    // the exit solves' exchange slots are the warp's, so two parts of it in
+    // the pass at once would overwrite each other's operands.  (FP32 EULERIAN
+    // exchanges nothing.)
+    const bool tracks = p >= 0 && !need_cell;
+    unsigned grp = 0u;
+    if constexpr (sizeof(R) == 8 || EXP) grp = __ballot_sync(FULL, tracks && V.passes < kMaxStepsPerVisit);
+    if (tracks) {
       R ox = zero, oy = zero, oz = zero;
       int r;
       if (++V.passes > kMaxStepsPerVisit) {
         r = PASS_UNDEFINED;
       } else {
-        r = rw_pass<R, EXP, AXI>(V, F, slots, massb, a.t_end, a.ndim, a.d1, a.d2, a.seed, id, ctr, ox, oy, oz);
+        r = rw_pass<R, EXP, AXI>(grp, V, F, slots, massb, a.t_end, a.ndim, a.d1, a.d2, a.seed, id, ctr, ox, oy, oz);
         if (EXP && r == PASS_WAIT) --V.passes;
         else ++my_passes;
       }
