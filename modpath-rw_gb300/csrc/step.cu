@@ -1565,12 +1565,21 @@ static size_t advance_smem_bytes(int threads, int exp_adv) {
   return (kRecUnits<R> * 16 + extra * sizeof(double)) * threads;
 }
 
+// A kernel's shared-memory limit is the process's, so it is the same at every
+// launch, whatever the block: a launch of few threads that lowered it to its
+// own size would have another host thread's launch of many refused.
+template <typename R, typename Kern>
+static cudaError_t raise_smem_limit(Kern kern, int exp_adv) {
+  const size_t most = advance_smem_bytes<R>(step_threads(sizeof(R) == 8, exp_adv != 0), exp_adv);
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 template <typename R>
 cudaError_t launch_advance(const AdvanceArgs<R> &a, int blocks, int threads, cudaStream_t s) {
   size_t smem = advance_smem_bytes<R>(threads, a.exp_adv);
   auto kern = a.exp_adv ? (a.axi ? rwpt_advance_kernel<R, true, true> : rwpt_advance_kernel<R, true, false>)
                         : (a.axi ? rwpt_advance_kernel<R, false, true> : rwpt_advance_kernel<R, false, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = raise_smem_limit<R>(kern, a.exp_adv);
   if (e != cudaSuccess) return e;
   kern<<<blocks, threads, smem, s>>>(a);
   return cudaGetLastError();
@@ -1581,7 +1590,7 @@ cudaError_t advance_occupancy(int exp_adv, int axi, int threads, int *blocks_per
   size_t smem = advance_smem_bytes<R>(threads, exp_adv);
   auto kern = exp_adv ? (axi ? rwpt_advance_kernel<R, true, true> : rwpt_advance_kernel<R, true, false>)
                       : (axi ? rwpt_advance_kernel<R, false, true> : rwpt_advance_kernel<R, false, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = raise_smem_limit<R>(kern, exp_adv);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, threads, smem);
 }
