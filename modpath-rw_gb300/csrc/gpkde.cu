@@ -830,27 +830,38 @@ __global__ void gather_x_kernel(KdeParams P, const SepPlan *pl, const T *val, Fi
 // 0.10; the multiply-adds bound them now.)  The order of the lists varies from
 // run to run; no element's value depends on it.
 //
-// A list holds a quarter of its buffer's elements.  Six fields per element
-// take six times the space, so that is enough for every plan of theirs; a plan
-// that flags more scans the mask instead.
+// A mask has a byte for every element its buffer could hold of one field; a
+// plan that uses fewer leaves the rest free, and the list lies there.  Six
+// fields per element take six times the space, so every plan of theirs has
+// room to list all its elements; a plan of one field that flags more than fit
+// scans the mask instead.
+struct Needed {
+  unsigned char *mask;
+  long long bytes;  // of the mask's allocation
+};
+__device__ __forceinline__ int *needed_list(const Needed &q, long long tot, long long &cap) {
+  const long long used = (tot + 15) / 16 * 16;  // (the masks are cleared, and read, past tot to a multiple of 8)
+  cap = used < q.bytes ? (q.bytes - used) / (long long)sizeof(int) : 0;
+  return reinterpret_cast<int *>(q.mask + used);
+}
 template <typename F>
-__device__ __forceinline__ void for_needed(long long tot, const unsigned char *mask, const int *list, long long n,
-                                           long long cap, F &&visit) {
+__device__ __forceinline__ void for_needed(long long tot, const Needed &q, long long n, F &&visit) {
+  long long cap;
+  const int *list = needed_list(q, tot, cap);
   const bool listed = n <= cap;
   const long long end = listed ? n : tot;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < end; i += (long long)gridDim.x * blockDim.x) {
     const long long g = listed ? (long long)list[i] : i;
-    if (listed || mask[g] != 0) visit(g);
+    if (listed || q.mask[g] != 0) visit(g);
   }
 }
 
 template <typename T, int NC>
 __global__ void __launch_bounds__(kThreads) gather_x_masked_kernel(KdeParams P, const SepPlan *pl, const T *val,
-                                                                  Fields<T> F, const unsigned char *mask,
-                                                                  const int *list, long long cap, T *T1) {
+                                                                  Fields<T> F, Needed q, T *T1) {
   __shared__ long long so[KDE_KMAX];
   const int np = load_offsets(pl, pl->o1, so);
-  for_needed(pl->tot1, mask, list, pl->n1, cap, [&](long long g) { gx_element<T, NC>(P, pl, val, F, T1, so, np, g); });
+  for_needed(pl->tot1, q, pl->n1, [&](long long g) { gx_element<T, NC>(P, pl, val, F, T1, so, np, g); });
 }
 
 // flag pass 2's elements at the bins' columns within mz of each bin
@@ -874,13 +885,15 @@ __global__ void mark_needed_kernel(KdeBinsT<T> B, const SepPlan *pl, const int *
 // before it along y flagged too, all but the last of these are that one's.
 constexpr int kListBytes = 4;
 template <bool DILATE>
-__global__ void __launch_bounds__(kThreads) list_needed_kernel(SepPlan *pl, const unsigned char *m, unsigned char *m1,
-                                                              int *list, long long cap) {
+__global__ void __launch_bounds__(kThreads) list_needed_kernel(SepPlan *pl, Needed q, unsigned char *m1) {
   __shared__ long long so[KDE_KMAX];
   __shared__ int item[kThreads * kListBytes], wsum[kThreads / 32];
   __shared__ long long first;
   const int np = load_offsets(pl, pl->o2, so);
   const long long tot = DILATE ? pl->tot2 : pl->tot1;
+  const unsigned char *m = q.mask;
+  long long cap;
+  int *list = needed_list(q, tot, cap);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (long long b = blockIdx.x * (long long)(kThreads * kListBytes); b < tot; b += (long long)gridDim.x * (kThreads * kListBytes)) {
     const long long e = b + threadIdx.x * kListBytes;
@@ -916,8 +929,8 @@ __global__ void __launch_bounds__(kThreads) list_needed_kernel(SepPlan *pl, cons
         const int my = pl->m[j][1];
         const bool prev = y > r2[2] && m[g - (r2[1] - r2[0] + 1)] != 0;
         const int y0 = max(r1[2], prev ? y + my : y - my), y1 = min(r1[3], y + my);
-        unsigned char *q = m1 + pl->o1[j];
-        for (int yy = y0; yy <= y1; ++yy) q[region_loc(r1, x, yy, z)] = 1;
+        unsigned char *mj = m1 + pl->o1[j];
+        for (int yy = y0; yy <= y1; ++yy) mj[region_loc(r1, x, yy, z)] = 1;
       }
     }
     __syncthreads();
@@ -1019,11 +1032,10 @@ __global__ void gather_y_kernel(KdeParams P, const SepPlan *pl, const T *val, co
 
 template <typename T, int NC>
 __global__ void __launch_bounds__(kThreads) gather_y_masked_kernel(KdeParams P, const SepPlan *pl, const T *val,
-                                                                  const T *T1, const unsigned char *mask,
-                                                                  const int *list, long long cap, T *T2) {
+                                                                  const T *T1, Needed q, T *T2) {
   __shared__ long long so[KDE_KMAX];
   const int np = load_offsets(pl, pl->o2, so);
-  for_needed(pl->tot2, mask, list, pl->n2, cap, [&](long long g) { gy_element<T, NC>(P, pl, val, T1, T2, so, np, g); });
+  for_needed(pl->tot2, q, pl->n2, [&](long long g) { gy_element<T, NC>(P, pl, val, T1, T2, so, np, g); });
 }
 
 // Gather pass 3 at every bin: sum_t fz[t] T2(bx, by, reflect(bz - m + t)).
@@ -1711,45 +1723,30 @@ cudaError_t KdeState::ensure_grid(int64_t ngrid) {
   return cudaSuccess;
 }
 
-// a list of needed elements: the passes do without (they scan the masks)
-// where the memory does not reach
-static int64_t alloc_list(int **p, int64_t n) {
-  if (cudaMalloc((void **)p, sizeof(int) * n) == cudaSuccess) return n;
-  (void)cudaGetLastError();
-  *p = nullptr;
-  return 0;
-}
-
 cudaError_t KdeState::ensure_pass(int64_t n1, int64_t n2) {
   if (n1 > t1_cap) {
     if (t1) cudaFree(t1);
     if (need1) cudaFree(need1);
-    if (list1) cudaFree(list1);
     t1 = nullptr;
     need1 = nullptr;
-    list1 = nullptr;
-    t1_cap = list1_cap = 0;
+    t1_cap = 0;
     const int64_t c = n1 + n1 / 4;
     cudaError_t e = cudaMalloc((void **)&t1, sizeof(double) * c);
     if (e == cudaSuccess) e = cudaMalloc((void **)&need1, c + 8);
     if (e != cudaSuccess) return e;
     t1_cap = c;
-    list1_cap = alloc_list(&list1, c / 4);
   }
   if (n2 > t2_cap) {
     if (t2) cudaFree(t2);
     if (need2) cudaFree(need2);
-    if (list2) cudaFree(list2);
     t2 = nullptr;
     need2 = nullptr;
-    list2 = nullptr;
-    t2_cap = list2_cap = 0;
+    t2_cap = 0;
     const int64_t c = n2 + n2 / 4;
     cudaError_t e = cudaMalloc((void **)&t2, sizeof(double) * c);
     if (e == cudaSuccess) e = cudaMalloc((void **)&need2, c + 8);
     if (e != cudaSuccess) return e;
     t2_cap = c;
-    list2_cap = alloc_list(&list2, c / 4);
   }
   return cudaSuccess;
 }
@@ -1758,7 +1755,7 @@ void KdeState::release() {
   void *ptrs[] = {bins.gx, bins.gy, bins.gz, bins.count, bins.ks, bins.scale, bins.shape, bins.support, bins.nest,
                   bins.dens, bins.cb, bins.rxx, bins.ryy, bins.rzz, bins.net, bins.dens_old, bins.scale_old,
                   partial, dens_grid, cx, cy, cz, d_scalars, d_flag, d_blockcnt, d_val, d_valf, d_meta, cell_bin,
-                  bin_key, d_keys, d_plan, t1, t2, need1, need2, list1, list2, d_wcnt, dens_raw, d_need, cxy, cxz, cyz, dens_out};
+                  bin_key, d_keys, d_plan, t1, t2, need1, need2, d_wcnt, dens_raw, d_need, cxy, cxz, cyz, dens_out};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (h_scalars) cudaFreeHost(h_scalars);
@@ -2051,20 +2048,21 @@ static cudaError_t kde_attempt(KdeState &st, const KdeParams &P, double hs, doub
   // and the launches as much: with lists 300,000 particles on 187 x 93 x 21
   // bins took 3.90 ms for 3.80.
   const bool masked = sizeof(T) == 8 && nb >= kMaskedBins && st.t1_cap < (int64_t)INT_MAX && st.t2_cap < (int64_t)INT_MAX;
+  const Needed needed1{st.need1, st.t1_cap + 8}, needed2{st.need2, st.t2_cap + 8};
   auto needed = [&](void) -> cudaError_t {
     if (!masked) return cudaSuccess;
     clear_needed_kernel<<<pgrid, kThreads, 0, s>>>(plan1, st.need1, st.need2);
     mark_needed_kernel<T><<<bb, kBinThreads, 0, s>>>(B, plan1, key1, st.need2);
-    list_needed_kernel<true><<<pgrid, kThreads, 0, s>>>(plan1, st.need2, st.need1, st.list2, st.list2_cap);
-    list_needed_kernel<false><<<pgrid, kThreads, 0, s>>>(plan1, st.need1, nullptr, st.list1, st.list1_cap);
+    list_needed_kernel<true><<<pgrid, kThreads, 0, s>>>(plan1, needed2, st.need1);
+    list_needed_kernel<false><<<pgrid, kThreads, 0, s>>>(plan1, needed1, nullptr);
     st.launches += 4;
     return cudaGetLastError();
   };
   auto gather_xy = [&](auto nc_tag, Fields<T> F) -> cudaError_t {
     constexpr int NC = decltype(nc_tag)::value;
     if (masked) {
-      gather_x_masked_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, F, st.need1, st.list1, st.list1_cap, t1);
-      gather_y_masked_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, t1, st.need2, st.list2, st.list2_cap, t2);
+      gather_x_masked_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, F, needed1, t1);
+      gather_y_masked_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, t1, needed2, t2);
     } else {
       gather_x_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, F, t1);
       gather_y_kernel<T, NC><<<pgrid, kThreads, 0, s>>>(P, plan1, val, t1, t2);

@@ -104,10 +104,9 @@ struct KdeState {
   SepPlan *d_plan = nullptr;
   double *t1 = nullptr, *t2 = nullptr;
   int64_t t1_cap = 0, t2_cap = 0;
-  // FP64 gathers: the elements of the passes that are read, as masks and lists
+  // FP64 gathers: the elements of the passes that are read, as masks (a byte per
+  // element of t1, t2, and 8) and, behind what a plan uses of them, lists
   unsigned char *need1 = nullptr, *need2 = nullptr;
-  int *list1 = nullptr, *list2 = nullptr;
-  int64_t list1_cap = 0, list2_cap = 0;
   double work_madds = 0;  // the last reconstruction's work model (multiply-adds of direct kernels)
   // run the optimisation loop as a device-side graph loop when the stream can
   // be captured; a batch's workers drive it from the host (several small
