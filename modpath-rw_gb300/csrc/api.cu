@@ -41,13 +41,15 @@ struct KdeWorker {
 };
 
 // The arrays of a flow time step as the caller gave them, kept between loads
-// (an array not given stays as it is; the step's view says which are).
+// (an array not given stays as it is; the step's view says which are).  Once
+// the records are made only IBOUNDTS, the retardation and the molecular
+// diffusion are read again; a load that is refused leaves those three alone.
 struct FlowRaw {
   int32_t *ia = nullptr, *ja = nullptr, *ibts = nullptr, *icb = nullptr, *ctype = nullptr, *zones = nullptr;
   double *flowja = nullptr, *bflow = nullptr, *por = nullptr, *ret = nullptr, *heads = nullptr, *src = nullptr;
   double *snk = nullptr, *aL = nullptr, *aT = nullptr, *dm = nullptr, *aLV = nullptr, *aTV = nullptr;
   int64_t nja_cap = 0;
-  size_t disp_cap = 0;
+  size_t disp_cap = 0, dm_cap = 0;
   void release() {
     for (void *p : {(void *)ia, (void *)ja, (void *)ibts, (void *)icb, (void *)ctype, (void *)zones, (void *)flowja,
                     (void *)bflow, (void *)por, (void *)ret, (void *)heads, (void *)src, (void *)snk, (void *)aL,
@@ -70,7 +72,7 @@ struct mprw_handle {
   double *d_colL = nullptr, *d_colR = nullptr, *d_rowF = nullptr, *d_rowB = nullptr, *d_sattop = nullptr;
   std::vector<double> h_top_cell;  // Top(n) after layer propagation
   // flow time step
-  FlowRaw flow, flow_next;            // in use, and the one a load fills and checks before it takes its place
+  FlowRaw flow;
   int32_t *d_ibts = nullptr;          // IBOUNDTS in use: flow.ibts, or a member's slice of the batch's array
   int *d_fflags = nullptr;            // what a load's check found (flow_check_kernel)
   CellBase base{};
@@ -223,7 +225,6 @@ void free_all(mprw_handle *h) {
   for (void *p : ptrs)
     if (p) cudaFree(p);
   h->flow.release();
-  h->flow_next.release();
   if (h->h_counters) cudaFreeHost(h->h_counters);
   if (h->h_abort) cudaFreeHost((void *)h->h_abort);
   if (h->d_counts) cudaFree(h->d_counts);
@@ -488,10 +489,11 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
   if (f->nja < nc || f->ia[0] != 1 || f->ia[nc] - 1 != f->nja)
     return fail(h, MPRW_E_INVAL, "mprw_load_flow: IA/JA inconsistent with the grid");
   const size_t nd = f->uniform_dispersion ? 1 : (size_t)nc;
-  // The step is uploaded beside the one in use, checked on the device and only
-  // then takes its place.  400,000 cells: the host's checks over 58 MB, the
-  // saturated tops and 24 allocations took 4.9 ms of a load, these 0.25.
-  FlowRaw &w = h->flow_next;
+  // The step is uploaded over the last one's arrays and checked on the device
+  // before the records are made from it.  400,000 cells: the host's checks over
+  // 58 MB, the saturated tops and 24 allocations took 4.9 ms of a load, these
+  // 0.25.
+  FlowRaw &w = h->flow;
   if (f->nja > w.nja_cap) {
     w.nja_cap = 0;
     CK(dalloc(&w.ja, f->nja));
@@ -499,37 +501,76 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
     w.nja_cap = f->nja;
   }
   if (nd > w.disp_cap) {
-    w.disp_cap = 0;
-    for (double **p : {&w.aL, &w.aT, &w.dm, &w.aLV, &w.aTV}) CK(dalloc(p, nd));
+    for (double **p : {&w.aL, &w.aT, &w.aLV, &w.aTV}) {
+      if (*p) cudaFree(*p);
+      *p = nullptr;
+    }
     w.disp_cap = nd;
   }
   cudaStream_t s = h->stream;
-  auto put = [s](auto **p, const auto *src, size_t count) -> cudaError_t {
+  auto put = [s](auto **p, const auto *src, size_t count, size_t cap) -> cudaError_t {
     if (!src) return cudaSuccess;
     if (!*p) {
-      const cudaError_t e = dalloc(p, count);
+      const cudaError_t e = dalloc(p, cap);
       if (e != cudaSuccess) return e;
     }
     return cudaMemcpyAsync(*p, src, sizeof(*src) * count, cudaMemcpyHostToDevice, s);
   };
-  CK(put(&w.ia, f->ia, nc + 1));
-  CK(put(&w.ja, f->ja, f->nja));
-  CK(put(&w.flowja, f->flowja, f->nja));
-  CK(put(&w.bflow, f->boundary_flows, 6 * nc));
-  CK(put(&w.por, f->porosity, nc));
-  CK(put(&w.ret, f->retardation, nc));
-  CK(put(&w.ibts, f->iboundts, nc));
-  CK(put(&w.icb, f->icboundts, nc));
-  CK(put(&w.heads, f->heads, nc));
-  CK(put(&w.ctype, f->celltype, nc));
-  CK(put(&w.src, f->source_flow, nc));
-  CK(put(&w.snk, f->sink_flow, nc));
-  CK(put(&w.zones, f->zones, nc));
-  CK(put(&w.aL, f->alpha_l, nd));
-  CK(put(&w.aT, f->alpha_t, nd));
-  CK(put(&w.dm, f->dm_eff, nd));
-  CK(put(&w.aLV, f->alpha_lv, nd));
-  CK(put(&w.aTV, f->alpha_tv, nd));
+  CK(put(&w.ia, f->ia, nc + 1, nc + 1));
+  CK(put(&w.ja, f->ja, f->nja, w.nja_cap));
+  CK(put(&w.flowja, f->flowja, f->nja, w.nja_cap));
+  CK(put(&w.bflow, f->boundary_flows, 6 * nc, 6 * nc));
+  CK(put(&w.por, f->porosity, nc, nc));
+  CK(put(&w.icb, f->icboundts, nc, nc));
+  CK(put(&w.heads, f->heads, nc, nc));
+  CK(put(&w.ctype, f->celltype, nc, nc));
+  CK(put(&w.src, f->source_flow, nc, nc));
+  CK(put(&w.snk, f->sink_flow, nc, nc));
+  CK(put(&w.zones, f->zones, nc, nc));
+  CK(put(&w.aL, f->alpha_l, nd, w.disp_cap));
+  CK(put(&w.aT, f->alpha_t, nd, w.disp_cap));
+  CK(put(&w.aLV, f->alpha_lv, nd, w.disp_cap));
+  CK(put(&w.aTV, f->alpha_tv, nd, w.disp_cap));
+  // The retardation and diffusion of a step that would take another's place
+  // wait in the scratch buffer for the checks' outcome (without the memory for
+  // it the host checks them).
+  auto put_kept = [&]() -> cudaError_t {
+    if (nd > w.dm_cap) {
+      w.dm_cap = 0;
+      const cudaError_t e = dalloc(&w.dm, nd);
+      if (e != cudaSuccess) return e;
+      w.dm_cap = nd;
+    }
+    const cudaError_t e = put(&w.ret, f->retardation, nc, nc);
+    return e != cudaSuccess ? e : put(&w.dm, f->dm_eff, nd, w.dm_cap);
+  };
+  const double *ret_new = nullptr, *dm_new = nullptr;
+  int bad = 0;
+  if (!h->flow_loaded) {
+    CK(put_kept());
+    ret_new = w.ret;
+    dm_new = w.dm;
+  } else {
+    const size_t ret_bytes = ((size_t)nc * 8 + 255) / 256 * 256, bytes = ret_bytes + nd * 8;
+    if (h->scratch_bytes < bytes) {
+      if (h->scratch) cudaFree(h->scratch);
+      h->scratch = nullptr;
+      h->scratch_bytes = 0;
+      if (cudaMalloc(&h->scratch, bytes) == cudaSuccess) h->scratch_bytes = bytes;
+      else (void)cudaGetLastError();
+    }
+    if (h->scratch) {
+      ret_new = (double *)h->scratch;
+      dm_new = (double *)((char *)h->scratch + ret_bytes);
+      CK(cudaMemcpyAsync(h->scratch, f->retardation, sizeof(double) * nc, cudaMemcpyHostToDevice, s));
+      CK(cudaMemcpyAsync((char *)h->scratch + ret_bytes, f->dm_eff, sizeof(double) * nd, cudaMemcpyHostToDevice, s));
+    } else {
+      for (int64_t c = 0; c < nc; ++c)
+        if (!(f->retardation[c] > 0.0) || !std::isfinite(f->retardation[c])) bad |= FLOW_BAD_POROSITY;
+      for (size_t c = 0; c < nd; ++c)
+        if (!std::isfinite(f->dm_eff[c])) bad |= FLOW_NON_FINITE;
+    }
+  }
   PrepInputs in{};
   in.g = h->g;
   in.delr = h->d_delr;
@@ -541,8 +582,7 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
   in.flowja = w.flowja;
   in.bflow = f->boundary_flows ? w.bflow : nullptr;
   in.porosity = w.por;
-  in.retardation = w.ret;
-  in.iboundts = w.ibts;
+  in.retardation = ret_new;
   in.icboundts = f->icboundts ? w.icb : nullptr;
   in.default_icbound = f->default_icbound;
   in.heads = f->heads ? w.heads : nullptr;
@@ -552,7 +592,7 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
   in.zones = f->zones ? w.zones : nullptr;
   in.alpha_l = w.aL;
   in.alpha_t = w.aT;
-  in.dm_eff = w.dm;
+  in.dm_eff = dm_new;
   in.alpha_lv = f->alpha_lv ? w.aLV : nullptr;
   in.alpha_tv = f->alpha_tv ? w.aTV : nullptr;
   in.dispersion_model = h->opt.dispersion_model;
@@ -571,9 +611,10 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
   if (!h->d_fflags) CK(cudaMalloc(&h->d_fflags, sizeof(int)));
   CK(cudaMemsetAsync(h->d_fflags, 0, sizeof(int), s));
   CK(launch_flow_check(in, f->nja, (int64_t)nd, h->d_fflags, s));
-  int bad = 0;
-  CK(cudaMemcpyAsync(&bad, h->d_fflags, sizeof(int), cudaMemcpyDeviceToHost, s));
+  int found = 0;
+  CK(cudaMemcpyAsync(&found, h->d_fflags, sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
+  bad |= found;
   if (bad & FLOW_BAD_POROSITY)
     return fail(h, MPRW_E_INVAL, "mprw_load_flow: porosity and retardation must be finite and > 0");
   if (bad & FLOW_NON_FINITE)
@@ -591,14 +632,24 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
       else CK(dalloc(&h->d_rec32, nc));
     }
   }
-  std::swap(h->flow, h->flow_next);
-  h->dm_uniform = f->uniform_dispersion != 0;
-  if (h->parent) {
-    CK(cudaMemcpyAsync(h->d_ibts, h->flow.ibts, sizeof(int32_t) * nc, cudaMemcpyDeviceToDevice, s));
-    in.iboundts = h->d_ibts;
-  } else {
-    h->d_ibts = h->flow.ibts;
+  // accepted: from here on it replaces the step in use
+  h->flow_loaded = false;
+  if (ret_new && ret_new != w.ret && nd <= w.dm_cap) {
+    CK(cudaMemcpyAsync(w.ret, ret_new, sizeof(double) * nc, cudaMemcpyDeviceToDevice, s));
+    CK(cudaMemcpyAsync(w.dm, dm_new, sizeof(double) * nd, cudaMemcpyDeviceToDevice, s));
+  } else if (ret_new != w.ret) {
+    CK(put_kept());
   }
+  h->dm_uniform = f->uniform_dispersion != 0;
+  if (!h->parent) {
+    CK(put(&w.ibts, f->iboundts, nc, nc));
+    h->d_ibts = w.ibts;
+  } else {
+    CK(cudaMemcpyAsync(h->d_ibts, f->iboundts, sizeof(int32_t) * nc, cudaMemcpyHostToDevice, s));
+  }
+  in.iboundts = h->d_ibts;
+  in.retardation = w.ret;
+  in.dm_eff = w.dm;
   // SaturatedTop (FlowModelData.f90:258-279) for ConvertToModelXYZ
   CK(launch_sattop(in, h->d_sattop, s));
   CK(cudaEventRecord(h->ev2, h->stream));

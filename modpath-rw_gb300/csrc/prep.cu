@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kRecThreads, 8) prep_rec_kernel(PrepInputs in,
 }
 
 // The checks a load makes before anything uses its arrays, in one pass over
-// them (bandwidth; the host took 4 ms over the same arrays).
+// those it was given (bandwidth; the host took 4 ms over the same arrays).
 __device__ __forceinline__ bool finite_bits(double v) {
   return (fb::bits(v) & 0x7FF0000000000000ULL) != 0x7FF0000000000000ULL;
 }
@@ -457,7 +457,7 @@ __global__ void flow_check_kernel(PrepInputs in, int64_t nja, int64_t ndisp, int
   all_finite(in.alpha_lv, ndisp);
   all_finite(in.alpha_tv, ndisp);
   for (int64_t i = i0; i < nc; i += step) {
-    const double p = in.porosity[i], r = in.retardation[i];
+    const double p = in.porosity[i], r = in.retardation ? in.retardation[i] : 1.0;
     if (!fb::above0(p) || !fb::above0(r) || !finite_bits(p) || !finite_bits(r)) bad |= FLOW_BAD_POROSITY;
     if (in.heads && fb::isnan_bits(in.heads[i])) bad |= FLOW_NAN_HEAD;
   }
