@@ -1644,7 +1644,7 @@ int mprw_gpkde(mprw_handle *h, const mprw_gpkde_options *o, double *density, dou
   if (rc != MPRW_OK) return rc;
   const int64_t ngrid = (int64_t)nb[0] * nb[1] * nb[2];
   // statistics of the active particles' coordinates (GridProjectedKDE.F90:4023-4030)
-  CK(h->kdep->ensure_grid(ngrid));
+  CK(h->kdep->ensure_grid(ngrid, s));
   double mean[3] = {0, 0, 0}, sd[3] = {0, 0, 0}, acc[4];
   rc = coord_sums(h, 0, nullptr, acc);
   if (rc != MPRW_OK) return rc;
@@ -1715,7 +1715,7 @@ int mprw_gpkde_from_counts(mprw_handle *h, const mprw_gpkde_options *o, const do
   CK(cudaEventRecord(h->ev2, s));
   const int64_t ngrid = (int64_t)nb[0] * nb[1] * nb[2];
   if (ensure_counts(h, ngrid) != MPRW_OK) return fail(h, MPRW_E_OOM, "mprw_gpkde_from_counts: device memory");
-  CK(h->kdep->ensure_grid(ngrid));
+  CK(h->kdep->ensure_grid(ngrid, s));
   CK(cudaMemcpyAsync(h->d_counts, mass_per_bin, sizeof(double) * ngrid, cudaMemcpyHostToDevice, s));
   // Kish effective mass of the summed weights (Histogram.F90:338-340); the
   // mass per bin becomes histogram%counts

@@ -1689,14 +1689,14 @@ cudaError_t KdeState::ensure_bins(int n) {
   return cudaSuccess;
 }
 
-cudaError_t KdeState::ensure_grid(int64_t ngrid) {
+cudaError_t KdeState::ensure_grid(int64_t ngrid, cudaStream_t s) {
   if (!d_scalars) {
     cudaError_t e = cudaMalloc((void **)&d_scalars, 32 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_wcnt, 64 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMallocHost((void **)&h_scalars, 96 * sizeof(double));  // + the 64 counters
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_flag, 2 * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(d_flag, 0, 2 * sizeof(int));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // (the handle's stream does not wait for it)
+    // (on the stream that uses them: the default one would wait for, and break, captures on blocking streams)
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_flag, 0, 2 * sizeof(int), s);
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_keys, sizeof(KeyAcc));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_plan, 2 * sizeof(SepPlan));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_need, 4 * sizeof(long long));

@@ -145,7 +145,7 @@ struct KdeState {
 
   cudaError_t ensure_bins(int n);
   cudaError_t ensure_pass(int64_t n1, int64_t n2);
-  cudaError_t ensure_grid(int64_t ngrid);
+  cudaError_t ensure_grid(int64_t ngrid, cudaStream_t s);
   void release();
 };
 
