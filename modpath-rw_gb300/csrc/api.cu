@@ -621,16 +621,16 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
     return fail(h, MPRW_E_INVAL, "mprw_load_flow: non-finite face flow, boundary flow, source/sink or dispersion value");
   if (bad & FLOW_NAN_HEAD) return fail(h, MPRW_E_INVAL, "mprw_load_flow: NaN head");
   if (bad & FLOW_BAD_JA) return fail(h, MPRW_E_INVAL, "mprw_load_flow: JA entry out of range");
-  if (!h->base.q) {
+  if (!h->d_massb) {  // (the last of them: after a failure all are made again)
     CK(dalloc(&h->base.q, 6 * nc));
     CK(dalloc(&h->base.dz, nc));
     CK(dalloc(&h->base.conn, 6 * nc));
-    CK(dalloc(&h->d_massb, nc));
     if (!h->parent) {  // a member's flags and records are slices of the batch's
       CK(dalloc(&h->base.flags, nc));
       if (h->opt.precision == MPRW_FP64) CK(dalloc(&h->d_rec64, nc));
       else CK(dalloc(&h->d_rec32, nc));
     }
+    CK(dalloc(&h->d_massb, nc));
   }
   // accepted: from here on it replaces the step in use
   h->flow_loaded = false;
@@ -682,6 +682,9 @@ int upload_particles(mprw_handle *h, int64_t n, const int32_t *cell, const doubl
   if (n > h->cap) {
     if (h->parent) return fail(h, MPRW_E_STATE, "batch member particle slice too small");
     size_t c = (size_t)n;
+    // until all are there the handle, and a batch's members, hold no particles
+    h->cap = h->n = 0;
+    for (mprw_handle *m : h->members) m->cap = m->n = 0;
     CK(dalloc(&h->d_cell, c));
     CK(dalloc(&h->d_status, c));
     CK(dalloc((char **)&h->d_x, c * rs));

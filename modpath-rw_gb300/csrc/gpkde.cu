@@ -1690,7 +1690,16 @@ cudaError_t KdeState::ensure_bins(int n) {
 }
 
 cudaError_t KdeState::ensure_grid(int64_t ngrid, cudaStream_t s) {
-  if (!d_scalars) {
+  if (!h_need) {  // (the last of them: after a failure all are made again)
+    for (void *p : {(void *)d_scalars, (void *)d_wcnt, (void *)d_flag, (void *)d_keys, (void *)d_plan, (void *)d_need})
+      if (p) cudaFree(p);
+    if (h_scalars) cudaFreeHost(h_scalars);
+    d_scalars = h_scalars = nullptr;
+    d_wcnt = nullptr;
+    d_flag = nullptr;
+    d_keys = nullptr;
+    d_plan = nullptr;
+    d_need = nullptr;
     cudaError_t e = cudaMalloc((void **)&d_scalars, 32 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_wcnt, 64 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMallocHost((void **)&h_scalars, 96 * sizeof(double));  // + the 64 counters

@@ -11,7 +11,7 @@ namespace {
 std::mutex g_mutex;
 std::unordered_map<void *, size_t> g_held;
 size_t g_live = 0, g_limit = (size_t)-1;
-long g_refused = 0;
+long g_refused = 0, g_refuse_in = 0;
 // (the runtime is loaded later, and not into the global scope)
 template <typename F>
 F next(const char *name) {
@@ -22,7 +22,8 @@ F next(const char *name) {
 extern "C" int cudaMalloc(void **p, size_t bytes) {
   static const auto real = next<int (*)(void **, size_t)>("cudaMalloc");
   std::lock_guard<std::mutex> lock(g_mutex);
-  if (bytes > g_limit || g_live > g_limit - bytes) {
+  const bool turn = g_refuse_in > 0 && --g_refuse_in == 0;
+  if (turn || bytes > g_limit || g_live > g_limit - bytes) {
     ++g_refused;
     *p = nullptr;
     return 2;  // cudaErrorMemoryAllocation
@@ -48,4 +49,6 @@ extern "C" int cudaFree(void *p) {
 
 extern "C" size_t malloc_limit_live() { return g_live; }
 extern "C" long malloc_limit_refused() { return g_refused; }
+// refuse the k-th call from here (1: the next) and no other; 0: none
+extern "C" void malloc_limit_refuse(long k) { g_refuse_in = k; }
 extern "C" void malloc_limit_set(size_t bytes) { g_limit = bytes; }

@@ -17,6 +17,7 @@ def limit():
     lib.malloc_limit_live.restype = ctypes.c_size_t
     lib.malloc_limit_refused.restype = ctypes.c_long
     lib.malloc_limit_set.argtypes = [ctypes.c_size_t]
+    lib.malloc_limit_refuse.argtypes = [ctypes.c_long]
     return lib
 
 
