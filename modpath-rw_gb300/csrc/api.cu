@@ -1007,7 +1007,9 @@ int launch_step(mprw_handle *h, double t_begin, double t_end, int bps, bool use_
   return MPRW_OK;
 }
 
-int sort_particles(mprw_handle *h) {
+// The processing order of an advance over [t_begin, t_end] at up to bps
+// resident blocks per SM.
+int sort_particles(mprw_handle *h, double t_begin, double t_end, int bps) {
   const uint64_t per_pass = 3ull * (uint64_t)h->ndim;  // Philox blocks per pass: 3 per normal, ndim normals
   PassGuess g{};
   if (h->opt.precision == MPRW_MIXED) {
@@ -1018,14 +1020,14 @@ int sort_particles(mprw_handle *h) {
     g.stride = sizeof(CellRec<double>);
   }
   g.t = h->d_t;
-  g.t_begin = h->last_t_begin;
-  g.t_end = h->last_t_end;
+  g.t_begin = t_begin;
+  g.t_end = t_end;
   // Heaviest first pays where warps take more than one round of particles; in
   // one round it only puts the long ones onto the same SMs (50,000 particles,
   // FP64, three intervals of five days: 1.9 1.7 1.6 ms by cell, 2.5 1.9 1.9
   // heaviest first).  EXPONENTIAL, whose long particles' solves slow each other
   // down, from two rounds on (10,000, 1.6 rounds: 11.3 against 12.2 ms).
-  const StepShape shape = step_shape(h, h->blocks_per_sm > 0 ? h->blocks_per_sm : default_blocks_per_sm(h));
+  const StepShape shape = step_shape(h, bps);
   const int64_t lanes = shape.blocks * (shape.threads / 32) * shape.lanes;
   const bool by_cell = h->n <= (h->opt.advection_kind == 1 ? 2 * lanes : lanes);
   CK(sort_cells(h->d_cell, by_cell ? nullptr : h->d_ctr, h->ctr_prev_valid ? h->d_ctr_prev : nullptr, per_pass, g, h->d_perm, h->n,
@@ -1064,10 +1066,11 @@ int mprw_advance(mprw_handle *h, double t_begin, double t_end, int64_t *steps_do
     if (steps_done) *steps_done = 0;
     return MPRW_OK;
   }
-  // sort the particles by cell every sort_interval-th advance; in between the
-  // last order is reused (the permutation stays valid while n is unchanged)
+  const int bps = h->blocks_per_sm > 0 ? h->blocks_per_sm : default_blocks_per_sm(h);
+  // sort the particles every sort_interval-th advance; in between the last
+  // order is reused (the permutation stays valid while n is unchanged)
   if (h->sort_interval > 0 && (h->advance_count % h->sort_interval == 0 || !h->perm_valid)) {
-    int rc = sort_particles(h);
+    int rc = sort_particles(h, t_begin, t_end, bps);
     if (rc != MPRW_OK) return rc;
   }
   ++h->advance_count;
@@ -1075,7 +1078,6 @@ int mprw_advance(mprw_handle *h, double t_begin, double t_end, int64_t *steps_do
     CK(cudaMemcpyAsync(h->d_ctr_prev, h->d_ctr, 8 * (size_t)h->n, cudaMemcpyDeviceToDevice, h->stream));
     h->ctr_prev_valid = true;
   }
-  const int bps = h->blocks_per_sm > 0 ? h->blocks_per_sm : default_blocks_per_sm(h);
   float ms = 0;
   int64_t steps = 0;
   int rc = launch_step(h, t_begin, t_end, bps, h->sort_interval > 0 && h->perm_valid, &ms, &steps);
@@ -1169,7 +1171,7 @@ int mprw_autotune(mprw_handle *h, double t_begin, double t_end, int32_t *blocks_
   for (int b = 1; b <= maxb; ++b) {
     CK(snapshot(true));
     CK(cudaEventRecord(h->ev2, s));
-    int rc = sort_particles(h);
+    int rc = sort_particles(h, t_begin, t_end, b);
     if (rc != MPRW_OK) return rc;
     float ms = 0, sort_ms = 0;
     int64_t st = 0;
