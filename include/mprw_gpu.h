@@ -396,23 +396,29 @@ int mprw_gpkde_batch(mprw_handle *batch, const mprw_gpkde_options *opts, double 
                      double *const *histogram, int32_t *loops_done, int32_t concurrency);
 
 /* Launch tuning of mprw_advance.  No counterpart in the reference (its loop
- * is `!$omp parallel do schedule(dynamic,1)`).  blocks_per_sm: resident
- * blocks per SM of the persistent step kernel (0 = the variant's default: 3
- * for EULERIAN MIXED, else 1; at most what its registers allow, which
- * mprw_get_tuning reports as max_blocks; blocks of 384 threads for the FP64
- * EULERIAN kernel, 256 otherwise); sort_interval: the particles are sorted
- * -- by the passes each took in the previous advance, heaviest first in
- * buckets of 8, then by cell -- before every k-th advance and processed in
- * that order until the next sort (1 = every advance, the default; 0 =
- * never).  Results do not depend on the tuning: each particle's steps use
- * only its own state and its own counter-based random numbers.
+ * is `!$omp parallel do schedule(dynamic,1)`).  blocks_per_sm: the most warps
+ * that the persistent step kernel keeps on an SM, in units of 12 for the FP64
+ * EULERIAN kernel and of 8 otherwise (0 = the variant's default: 3 for EULERIAN
+ * MIXED, else 1; at most what its registers allow, which mprw_get_tuning
+ * reports as max_blocks).  Where the particles do not fill them a launch takes
+ * fewer -- FP64 EULERIAN up to 128 particles per SM four at most, MIXED up to
+ * 256 eight, EXPONENTIAL below 80,000 particles four -- so for few particles
+ * the setting may change nothing.  sort_interval: the particles are sorted --
+ * heaviest first in buckets of four expected passes (those of the previous
+ * advance, or the time left over the cell's time step), then by cell; by cell
+ * alone where one round of the launch's lanes, EXPONENTIAL two, takes them all
+ * -- before every k-th advance and processed in that order until the next sort
+ * (1 = every advance, the default; 0 = never).  Results do not depend on the
+ * tuning: each particle's steps use only its own state and its own
+ * counter-based random numbers.
  *
  * mprw_autotune picks both on the handle's real work: from the current
  * particle state it runs one advance over [t_begin, t_end] per candidate
  * (sorted first, with 1 .. min(max_blocks, 4) blocks per SM, then the best
  * block count unsorted), restoring the state before each trial and at the
  * end, so the particles are unchanged on return.  The fastest block count
- * (particle-steps per ms, sort included) is kept; sorting is kept every
+ * (particle-steps per ms, sort included) is kept, the default where it gives
+ * the same launch; sorting is kept every
  * advance if it pays, every 4th if unsorted is within 3 %, never if unsorted
  * is more than 5 % faster.  rates (may be NULL; room for 5 doubles) receives
  * the particle-steps per ms of each trial in that order.  Costs one extra

@@ -862,6 +862,7 @@ int default_blocks_per_sm(mprw_handle *h) {
 struct StepShape {
   int threads, lanes;  // threads per block; lanes of each warp that take particles
   int64_t blocks;
+  bool operator==(const StepShape &o) const { return threads == o.threads && lanes == o.lanes && blocks == o.blocks; }
 };
 
 // Many particles fill every resident warp.  With fewer, the kernel ends with
@@ -1187,6 +1188,9 @@ int mprw_autotune(mprw_handle *h, double t_begin, double t_end, int32_t *blocks_
       rate_sorted = r;
     }
   }
+  // few particles take the same launch at several counts, and their trials
+  // differ by chance alone: the default then
+  if (step_shape(h, best_b) == step_shape(h, default_blocks_per_sm(h))) best_b = default_blocks_per_sm(h);
   // the same without sorting: the particles in the order the caller gave
   CK(snapshot(true));
   float ms_u = 0;
