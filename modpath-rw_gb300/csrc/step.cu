@@ -16,6 +16,8 @@
 // TrackCell (TrackCell.f90:375-669) and ConvertFromNeighbor
 // (RectangularGridDisMf6.f90:50-108).  Interpolants are evaluated from the
 // monomial coefficients the prep kernel stores, with fused multiply-adds.
+#include <cstddef>
+
 #include "mprw_common.cuh"
 #include "mprw_kernels.cuh"
 #include "nrscan.cuh"
@@ -118,6 +120,20 @@ template <typename R>
 constexpr int kRecUnits = sizeof(R) == 8 ? 33 : 17;
 template <typename R>
 constexpr int kRecStride = kRecUnits<R> * 16 / (int)sizeof(R);
+// The copies take the record's bytes as they lie, so the fields' numbers are
+// its layout.
+template <typename R>
+constexpr bool layout_is_the_records() {
+  using C = CellRec<R>;
+  constexpr size_t r = sizeof(R);
+  return offsetof(C, v1) == F_V1 * r && offsetof(C, dv) == F_DV * r && offsetof(C, d) == F_D * r &&
+         offsetof(C, inv_d) == F_INVD * r && offsetof(C, div) == F_DIV * r && offsetof(C, vb) == F_VB * r &&
+         offsetof(C, aL) == F_AL * r && offsetof(C, aT) == F_AT * r && offsetof(C, dm) == F_DM * r &&
+         offsetof(C, two_over_r) == F_2R * r && offsetof(C, v2) == F_V2 * r && offsetof(C, aLV) == F_ALV * r &&
+         offsetof(C, aTV) == F_ATV * r && sizeof(C) % 16 == 0 && alignof(C) >= 16 &&
+         sizeof(C) >= 16 * kRecUnits<R> && NFIELDS * r <= 16 * kRecUnits<R>;
+}
+static_assert(layout_is_the_records<double>() && layout_is_the_records<float>(), "CellRec moved: renumber the fields");
 
 // Asynchronous copies, all in flight at once and without a register each;
 // stage_wait before the first read.  Every warp waits here for its entering
