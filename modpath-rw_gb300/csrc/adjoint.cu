@@ -27,6 +27,7 @@
 #include <string>
 
 #include "adjoint.cuh"
+#include "dispadj.cuh"
 
 namespace mprw {
 
@@ -172,9 +173,6 @@ __global__ void adj_node_div_kernel(AdjGrid G, const double *phi, const double *
 // cell size that is a power of two (exact): 145 and 430 instructions, 100,000
 // particles 1.03 -> 0.59 ms and 3.18 -> 1.83 ms per 20 steps (84 % active).
 __device__ __forceinline__ double sqrt_i(double x) { return fb::sqrt_plain(x) ? fb::sqrt_core(x) : sqrt(x); }
-__device__ __forceinline__ double div_i(double a, double b) {
-  return fb::div_plain(a, b) ? fb::div_core(a, b, 0) : a / b;
-}
 
 // The cell of a position and its local coordinates (the position is inside
 // the domain after the fold; the last cell takes the upper face).
@@ -258,10 +256,6 @@ __device__ __forceinline__ void interp(const AdjGrid &G, const double *nodes, co
     I.dm += w * nd.v[8];
   }
 }
-
-struct Disp {
-  double s2, r, a, b, kappa, P, bxi[3];
-};
 
 // B xi = a xi + kappa (u . xi) u
 __device__ __forceinline__ void displacement(const AdjGrid &G, const Interp &I, const double xi[3], Disp &D) {
@@ -433,32 +427,9 @@ __device__ __forceinline__ void step_reverse(const AdjGrid &G, const double *nod
     (void)fold(y, G.lo[d], G.n[d] * G.d[d], sg);
     lt[d] = fb::below0(sg) ? -lam[d] : lam[d];
   }
-  // B xi = a xi + kappa P u as a function of u, aL, aT, dm: the transposed
-  // derivatives applied to lt.  With r = sqrt(|u|^2 + eps^2): da = (aT / a)
-  // dr, dr = (u . du) / r, db = d(ll) / b, dkappa = -kappa (dr / r + (da + db)
-  // / (a + b)).  Four reciprocals serve every quotient.
-  const double ul = I.u[0] * lt[0] + I.u[1] * lt[1] + I.u[2] * lt[2];
-  const double xl = xi[0] * lt[0] + xi[1] * lt[1] + xi[2] * lt[2];
-  const double k = D.kappa, P = D.P, s2 = D.s2, dA = I.aL - I.aT;
-  const double ir = div_i(1.0, D.r), ia = div_i(1.0, D.a), ib = div_i(1.0, D.b), iab = div_i(1.0, D.a + D.b);
-  const double ir2 = ir * ir, s2r = s2 * ir;
-  const double ca = I.aT * ia * ir;                                          // da = ca (u . du)
-  const double cb = (I.aT * ir + dA * (2.0 * ir - s2r * ir2)) * ib;          // db = cb (u . du)
-  const double ck = -k * (ir2 + (ca + cb) * iab);                            // dkappa = ck (u . du)
-  const double Pul = P * ul, ju = ca * xl + ck * Pul, jx = k * ul, jl = k * P;
-  const double da_daT = D.r * ia, db_daT = (D.r - s2r) * ib;
-  const double cL = ir * iab * (2.0 - k * s2 * ib) * Pul;
-  const double cT = da_daT * xl - iab * (2.0 * ir + k * (da_daT + db_daT)) * Pul;
-  const double cD = xl * ia - k * (ia + ib) * iab * Pul;
   // dL/d(field) of the interpolated u, G, aL, aT, Dm
   double q[9];
-  for (int d = 0; d < 3; ++d) {
-    q[3 + d] = dt * lt[d];
-    q[d] = q[3 + d] + sdt * (ju * I.u[d] + jx * xi[d] + jl * lt[d]);
-  }
-  q[6] = sdt * cL;
-  q[7] = sdt * cT;
-  q[8] = sdt * cD;
+  displacement_adjoint(D, I.u, I.aL, I.aT, xi, lt, dt, sdt, q);
   double s[8];  // per corner: q . node values
 #pragma unroll
   for (int o = 0; o < 8; ++o) {
