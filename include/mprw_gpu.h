@@ -402,7 +402,7 @@ int mprw_gpkde_batch(mprw_handle *batch, const mprw_gpkde_options *opts, double 
  * MIXED, else 1; at most what its registers allow, which mprw_get_tuning
  * reports as max_blocks).  Where the particles do not fill them a launch takes
  * fewer -- FP64 EULERIAN up to 128 particles per SM four at most, MIXED up to
- * 256 eight, EXPONENTIAL below 80,000 particles four -- so for few particles
+ * 256 eight, EXPONENTIAL up to 526 four -- so for few particles
  * the setting may change nothing.  sort_interval: the particles are sorted --
  * heaviest first in buckets of four expected passes (those of the previous
  * advance, or the time left over the cell's time step), then by cell; by cell

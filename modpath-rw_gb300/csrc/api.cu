@@ -849,8 +849,8 @@ int max_blocks_per_sm(mprw_handle *h) {
   return nb;
 }
 
-// EXPONENTIAL: particles from which every resident warp is filled
-constexpr int64_t kExpSpread = 80000;
+// EXPONENTIAL: the most particles per SM that are spread over few warps
+constexpr int64_t kExpSpread = 526;
 
 int default_blocks_per_sm(mprw_handle *h) {
   // EULERIAN MIXED is compiled for 3 resident blocks per SM (80 registers)
@@ -875,9 +875,13 @@ struct StepShape {
 // (ms, all warps full -> spread): FP64 column of 2,000 particles 2.39 -> 1.15,
 // 30,000: 2.55 -> 1.80; FP64 100x60x10 field, 4,000: 8.35 -> 5.77, 16,000: 9.29
 // -> 7.0; MIXED, 4,000: 3.23 -> 1.97; EXPONENTIAL, 61x37x7 field, 4,000: 13.3 ->
-// 8.2 (one interval), 40,000: 37.4 -> 30.4, 80,000: 24.1 and 24.7 (one interval),
-// 150,000: 36.8 filled, 41.2 spread (first intervals in cell order; 21.8 and 34.2
-// heaviest first).  Past one particle per lane the FP64 warps are levelled
+// 8.2 (one interval), 40,000: 37.4 -> 30.4.  Where EXPONENTIAL fills every warp
+// depends on the field: first intervals of five days, heaviest first, spread
+// and filled, in the 61x37x7 field 60,000 18.6 and 19.9, 80,000 22.6 and 22.1,
+// 150,000 40.1 and 35.0 (MIXED 17.7 and 18.7, 22.0 and 20.1, 38.4 and 31.7); in a
+// 100x60x10 one 80,000 30.2 and 41.0, 100,000 32.3 and 41.2, 150,000 44.1 and 45.6,
+// third intervals 26.6 and 28.3 at 100,000, 38.3 and 33.9 at 150,000.  The line is
+// the first field's.  Past one particle per lane the FP64 warps are levelled
 // over the rounds (100,000 particles, 12 warps -> 11: 7.07 -> 6.71); MIXED runs
 // blocks of four warps (1,000,000: equal; 40,000 in the column: 0.78 -> 0.70).
 StepShape step_shape(mprw_handle *h, int bps) {
@@ -889,8 +893,8 @@ StepShape step_shape(mprw_handle *h, int bps) {
   int64_t warps, lanes = 32;  // warps per SM
   if (exp_adv) {
     // Newton's passes differ most between particles: 0.6 lanes per particle
-    warps = h->n < kExpSpread ? 4 : max_warps;
-    if (h->n < kExpSpread) lanes = ceil_div(6 * per, 40);
+    warps = per <= kExpSpread ? 4 : max_warps;
+    if (per <= kExpSpread) lanes = ceil_div(6 * per, 40);
   } else if (mixed) {
     warps = per <= 256 ? 8 : max_warps;
     lanes = ceil_div(per, 8);
@@ -1027,7 +1031,10 @@ int sort_particles(mprw_handle *h, double t_begin, double t_end, int bps) {
   // one round it only puts the long ones onto the same SMs (50,000 particles,
   // FP64, three intervals of five days: 1.9 1.7 1.6 ms by cell, 2.5 1.9 1.9
   // heaviest first).  EXPONENTIAL, whose long particles' solves slow each other
-  // down, from two rounds on (10,000, 1.6 rounds: 11.3 against 12.2 ms).
+  // down, from two rounds on (first intervals by cell and heaviest first: in the
+  // 61x37x7 field 10,000 10.9 and 10.7 ms, 20,000 13.4 and 13.1, 40,000 15.5 and
+  // 14.9, 60,000 19.9 and 18.6; in a 100x60x10 one 18.2 and 20.3, 24.5 and 25.2, 23.4
+  // and 29.6, 29.8 and 29.9; in the intervals after them 3 % for the latter).
   const StepShape shape = step_shape(h, bps);
   const int64_t lanes = shape.blocks * (shape.threads / 32) * shape.lanes;
   const bool by_cell = h->n <= (h->opt.advection_kind == 1 ? 2 * lanes : lanes);
