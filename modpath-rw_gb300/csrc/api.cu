@@ -531,9 +531,9 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
   CK(put(&w.aT, f->alpha_t, nd, w.disp_cap));
   CK(put(&w.aLV, f->alpha_lv, nd, w.disp_cap));
   CK(put(&w.aTV, f->alpha_tv, nd, w.disp_cap));
-  // The retardation and diffusion of a step that would take another's place
-  // wait in the scratch buffer for the checks' outcome (without the memory for
-  // it the host checks them).
+  // IBOUNDTS, retardation and diffusion of a step that would take another's
+  // place wait in the scratch buffer for the checks' outcome (without the
+  // memory for it the host checks them).
   auto put_kept = [&]() -> cudaError_t {
     if (nd > w.dm_cap) {
       w.dm_cap = 0;
@@ -541,17 +541,21 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
       if (e != cudaSuccess) return e;
       w.dm_cap = nd;
     }
-    const cudaError_t e = put(&w.ret, f->retardation, nc, nc);
-    return e != cudaSuccess ? e : put(&w.dm, f->dm_eff, nd, w.dm_cap);
+    cudaError_t e = put(&w.ret, f->retardation, nc, nc);
+    if (e == cudaSuccess) e = put(&w.dm, f->dm_eff, nd, w.dm_cap);
+    if (e == cudaSuccess) e = put(h->parent ? &h->d_ibts : &w.ibts, f->iboundts, nc, nc);  // (a member's is there)
+    return e;
   };
   const double *ret_new = nullptr, *dm_new = nullptr;
+  const int32_t *ibts_new = nullptr;
   int bad = 0;
   if (!h->flow_loaded) {
     CK(put_kept());
     ret_new = w.ret;
     dm_new = w.dm;
   } else {
-    const size_t ret_bytes = ((size_t)nc * 8 + 255) / 256 * 256, bytes = ret_bytes + nd * 8;
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t dm_at = up(8 * (size_t)nc), ibts_at = dm_at + up(8 * nd), bytes = ibts_at + 4 * (size_t)nc;
     if (h->scratch_bytes < bytes) {
       if (h->scratch) cudaFree(h->scratch);
       h->scratch = nullptr;
@@ -560,10 +564,13 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
       else (void)cudaGetLastError();
     }
     if (h->scratch) {
-      ret_new = (double *)h->scratch;
-      dm_new = (double *)((char *)h->scratch + ret_bytes);
-      CK(cudaMemcpyAsync(h->scratch, f->retardation, sizeof(double) * nc, cudaMemcpyHostToDevice, s));
-      CK(cudaMemcpyAsync((char *)h->scratch + ret_bytes, f->dm_eff, sizeof(double) * nd, cudaMemcpyHostToDevice, s));
+      char *b = (char *)h->scratch;
+      ret_new = (double *)b;
+      dm_new = (double *)(b + dm_at);
+      ibts_new = (int32_t *)(b + ibts_at);
+      CK(cudaMemcpyAsync(b, f->retardation, sizeof(double) * nc, cudaMemcpyHostToDevice, s));
+      CK(cudaMemcpyAsync(b + dm_at, f->dm_eff, sizeof(double) * nd, cudaMemcpyHostToDevice, s));
+      CK(cudaMemcpyAsync(b + ibts_at, f->iboundts, sizeof(int32_t) * nc, cudaMemcpyHostToDevice, s));
     } else {
       for (int64_t c = 0; c < nc; ++c)
         if (!(f->retardation[c] > 0.0) || !std::isfinite(f->retardation[c])) bad |= FLOW_BAD_POROSITY;
@@ -634,19 +641,15 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
   }
   // accepted: from here on it replaces the step in use
   h->flow_loaded = false;
-  if (ret_new && ret_new != w.ret && nd <= w.dm_cap) {
+  if (ibts_new && nd <= w.dm_cap) {
     CK(cudaMemcpyAsync(w.ret, ret_new, sizeof(double) * nc, cudaMemcpyDeviceToDevice, s));
     CK(cudaMemcpyAsync(w.dm, dm_new, sizeof(double) * nd, cudaMemcpyDeviceToDevice, s));
+    CK(cudaMemcpyAsync(h->d_ibts, ibts_new, sizeof(int32_t) * nc, cudaMemcpyDeviceToDevice, s));
   } else if (ret_new != w.ret) {
     CK(put_kept());
   }
+  if (!h->parent) h->d_ibts = w.ibts;
   h->dm_uniform = f->uniform_dispersion != 0;
-  if (!h->parent) {
-    CK(put(&w.ibts, f->iboundts, nc, nc));
-    h->d_ibts = w.ibts;
-  } else {
-    CK(cudaMemcpyAsync(h->d_ibts, f->iboundts, sizeof(int32_t) * nc, cudaMemcpyHostToDevice, s));
-  }
   in.iboundts = h->d_ibts;
   in.retardation = w.ret;
   in.dm_eff = w.dm;
