@@ -641,20 +641,15 @@ int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *f) {
   }
   // accepted: from here on it replaces the step in use
   h->flow_loaded = false;
-  if (ibts_new && nd <= w.dm_cap) {
-    CK(cudaMemcpyAsync(w.ret, ret_new, sizeof(double) * nc, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(w.dm, dm_new, sizeof(double) * nd, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(h->d_ibts, ibts_new, sizeof(int32_t) * nc, cudaMemcpyDeviceToDevice, s));
-  } else if (ret_new != w.ret) {
-    CK(put_kept());
-  }
+  HeldBack held{};
+  if (ibts_new && nd <= w.dm_cap) held = {ret_new, dm_new, ibts_new, (int64_t)nd};
+  else if (ret_new != w.ret) CK(put_kept());
   if (!h->parent) h->d_ibts = w.ibts;
   h->dm_uniform = f->uniform_dispersion != 0;
   in.iboundts = h->d_ibts;
   in.retardation = w.ret;
   in.dm_eff = w.dm;
-  // SaturatedTop (FlowModelData.f90:258-279) for ConvertToModelXYZ
-  CK(launch_sattop(in, h->d_sattop, s));
+  CK(launch_take(in, held, w.ret, w.dm, h->d_ibts, h->d_sattop, s));
   CK(cudaEventRecord(h->ev2, h->stream));
   CK(launch_prep(in, h->base, h->d_massb, h->d_rec64, h->d_rec32, h->stream));
   if (h->cell0 != 0) {

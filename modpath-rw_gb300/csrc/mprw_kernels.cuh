@@ -67,7 +67,17 @@ struct PrepInputs {
 // what a flow time step's check found (bits of *flag)
 enum : int { FLOW_BAD_POROSITY = 1, FLOW_NON_FINITE = 2, FLOW_NAN_HEAD = 4, FLOW_BAD_JA = 8 };
 cudaError_t launch_flow_check(const PrepInputs &in, int64_t nja, int64_t ndisp, int *flag, cudaStream_t s);
-cudaError_t launch_sattop(const PrepInputs &in, double *sattop, cudaStream_t s);
+// The arrays of an accepted step that were held back from the step in use
+// (each null: in place already); dm has ndisp values.
+struct HeldBack {
+  const double *ret, *dm;
+  const int32_t *ibts;
+  int64_t ndisp;
+};
+// SaturatedTop, and the arrays held back to their places (in.retardation,
+// in.dm_eff, in.iboundts)
+cudaError_t launch_take(const PrepInputs &in, const HeldBack &held, double *ret, double *dm, int32_t *ibts,
+                        double *sattop, cudaStream_t s);
 cudaError_t launch_prep(const PrepInputs &in, CellBase base, uint8_t *massb, CellRec<double> *rec64,
                         CellRec<float> *rec32, cudaStream_t s);
 

@@ -471,21 +471,28 @@ cudaError_t launch_flow_check(const PrepInputs &in, int64_t nja, int64_t ndisp, 
   return cudaGetLastError();
 }
 
-// SaturatedTop of every cell (FlowModelData.f90:258-279): the head of an
-// active convertible cell that holds it, else the cell's top
-__global__ void sattop_kernel(PrepInputs in, double *sattop) {
+// An accepted step takes its place: SaturatedTop of every cell
+// (FlowModelData.f90:258-279), the head of an active convertible cell that
+// holds it, else the cell's top; and the arrays held back until now (as copies
+// of their own they cost a load 20 us of host calls).
+__global__ void take_kernel(PrepInputs in, HeldBack held, double *ret, double *dm, int32_t *ibts, double *sattop) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= in.g.ncell) return;
+  const int32_t ib = held.ibts ? held.ibts[n] : ibts[n];
+  if (held.ibts) ibts[n] = ib;
+  if (held.ret) ret[n] = held.ret[n];
+  if (held.dm && n < held.ndisp) dm[n] = held.dm[n];
   double t = n < in.g.ncpl ? in.top[n] : in.botm[n - in.g.ncpl];
-  if (in.celltype && in.heads && in.celltype[n] == 1 && in.iboundts[n] != 0) {
+  if (in.celltype && in.heads && in.celltype[n] == 1 && ib != 0) {
     const double hd = in.heads[n];
     if (hd <= t && hd >= in.botm[n]) t = hd;
   }
   sattop[n] = t;
 }
 
-cudaError_t launch_sattop(const PrepInputs &in, double *sattop, cudaStream_t s) {
-  sattop_kernel<<<(in.g.ncell + 255) / 256, 256, 0, s>>>(in, sattop);
+cudaError_t launch_take(const PrepInputs &in, const HeldBack &held, double *ret, double *dm, int32_t *ibts,
+                        double *sattop, cudaStream_t s) {
+  take_kernel<<<(in.g.ncell + 255) / 256, 256, 0, s>>>(in, held, ret, dm, ibts, sattop);
   return cudaGetLastError();
 }
 
