@@ -2052,8 +2052,8 @@ static cudaError_t kde_attempt(KdeState &st, const KdeParams &P, double hs, doub
   // an int (the pass capacity bounds them).  From 16,384 active bins: below,
   // the four launches that find the elements take longer than the elements
   // left out (ms per reconstruction of 8 loops without and with them: 3,171
-  // bins 1.66 and 1.90, 6,607 1.90 and 2.10, 11,200 2.24 and 2.40, 24,191 3.42
-  // and 3.25, 56,392 7.38 and 6.15).  FP32's multiply-adds cost a sixteenth
+  // bins 1.58 and 1.85, 6,607 1.84 and 2.02, 11,200 2.15 and 2.34, 24,191 3.29
+  // and 3.13, 56,392 7.21 and 6.00).  FP32's multiply-adds cost a sixteenth
   // and the launches as much: with lists 300,000 particles on 187 x 93 x 21
   // bins took 3.90 ms for 3.80.
   const bool masked = sizeof(T) == 8 && nb >= kMaskedBins && st.t1_cap < (int64_t)INT_MAX && st.t2_cap < (int64_t)INT_MAX;
@@ -2165,9 +2165,9 @@ static cudaError_t kde_attempt(KdeState &st, const KdeParams &P, double hs, doub
   KCK(reduce(RED_ALMISE));  // nEstimate and net roughness are zero: 0
   // A conditional graph takes some 0.25 ms to build, more than the host's read
   // after each of the few loops a small reconstruction runs; the host-driven
-  // loop's graph is kept and updated.  (ms, device and host: 7 bins 0.53 and
-  // 0.47, 1,459 bins 2.00 and 1.98, 3,171 bins 1.66 and 1.65, 56,392 bins both
-  // 7.38 -- there the host's reads would only tie up its thread.)
+  // loop's graph is kept and updated.  (ms, device and host: 7 bins 0.54 and
+  // 0.48, 1,459 bins 1.97 and 1.93, 3,171 bins 1.64 and 1.58, 11,200 2.16 and 2.13,
+  // 56,392 6.01 and 5.99 -- there the host's reads would only tie up its thread.)
   if (n_opt_loops > 0 && st.device_loop && nb >= kDeviceLoopBins) {
     // the whole loop as one graph: a while node around the captured body (a
     // while node runs its body at least once: no loops are the host path's)
