@@ -119,7 +119,9 @@ typedef struct {
 int mprw_create(mprw_handle **h, const mprw_grid_desc *grid, const mprw_options *opt);
 
 /* Upload one flow time step and build the per-cell records on the device.
- * Replaces the per-cell-entry buffer fills listed in the header comment. */
+ * Replaces the per-cell-entry buffer fills listed in the header comment.  A
+ * step refused with MPRW_E_INVAL leaves the one before it in use; a failure
+ * of the device later than that leaves the handle without a step. */
 int mprw_load_flow(mprw_handle *h, const mprw_flow_desc *flow);
 
 /* Copy n particles (host arrays) to the device.  cell is 1-based; t is the
